@@ -399,17 +399,12 @@ extern "C" {
 // ---------------------------------------------------------------------------
 // sigma_min (svdvals(A)[end], macros.jl:159-161) for every k: the k are taken
 // in chunks; a chunk's A(k) are assembled in FP64 straight into one LU batch,
-// factored by the library's batched LU and inverted (LU solves with the
-// identity), and the subspace iteration on the inverses runs on the device
-// until 1/sqrt(lambda_max) changes by less than 1e-13 relative (at most
-// SM_ITERS steps): for many operators of n <= 1024 one CTA per k runs the
-// whole iteration and one host synchronisation per chunk reads the results;
-// otherwise each k's products are split over the whole GPU (sigma_single).
-// An exactly singular U gives sigma_min = 0.
+// factored by the library's batched LU, and one launch runs the whole Lanczos
+// iteration on the factors (sigma_lu); one host synchronisation at the end
+// reads the results. An exactly singular U gives sigma_min = 0.
 // ---------------------------------------------------------------------------
 qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig) {
   if (!g || !ks || !sig || nk < 1) { set_error("qbg_sigma_min: invalid arguments"); return QBG_EINVAL; }
-  constexpr int SM_ITERS = 40;
   std::vector<double> kc(2 * nk);
   for (int64_t q = 0; q < nk; ++q) { kc[2 * q] = ks[q]; kc[2 * q + 1] = 0.0; }
   QBG_TRY(check_ks(kc.data(), nk));
@@ -440,60 +435,33 @@ qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig)
       cudaEventDestroy(e);
     }
   } sguard{st, ev_in};
-  // chunk: the operators and their inverses within about 1 GB
-  const size_t per_k = sizeof(cxd) * (size_t)n * n * 2;
+  // chunk: the operators within about 1 GB
+  const size_t per_k = sizeof(cxd) * (size_t)n * n;
   const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nk, 256),
                                                                 (int64_t)((1ull << 30) / per_k)));
   int s = QBG_OK;
   {
     Dense64 D;
-    cxd *Cinv = nullptr, *dks = nullptr, *work = nullptr, *X0 = nullptr, *CH = nullptr, *P = nullptr;
-    double *dsig = nullptr, *state = nullptr;
+    cxd *dks = nullptr, *work = nullptr;
+    double* dsig = nullptr;
     void** dptrs = nullptr;
-    // many small operators: one CTA per k runs the whole iteration (sigma_iterate);
-    // otherwise each k's products are spread over the GPU (sigma_single)
-    const bool per_cta = n <= 1024 && chunk >= 16;
-    if ((s = D.create(n, chunk, st)) || (s = D.alloc(&Cinv, sizeof(cxd) * (size_t)n * n * chunk)) ||
-        (s = D.alloc(&dks, sizeof(cxd) * nk)) || (s = D.alloc(&work, sizeof(cxd) * (size_t)3 * n * DENSE_P * chunk)) ||
-        (s = D.alloc(&X0, sizeof(cxd) * (size_t)n * DENSE_P)) || (s = D.alloc(&dsig, sizeof(double) * chunk)) ||
-        (s = D.alloc(&dptrs, sizeof(void*) * chunk)) ||
-        (!per_cta && ((s = D.alloc(&CH, sizeof(cxd) * (size_t)n * n)) ||
-                      (s = D.alloc(&P, sizeof(cxd) * std::max<size_t>(gemm_tall_scratch(n, DENSE_P), 1))) ||
-                      (s = D.alloc(&state, sizeof(double) * (2 + 2 * DENSE_P))))))
+    if ((s = D.create(n, chunk, st)) || (s = D.alloc(&dks, sizeof(cxd) * nk)) ||
+        (s = D.alloc(&work, sizeof(cxd) * sigma_lu_work(n) * chunk)) || (s = D.alloc(&dsig, sizeof(double) * nk)) ||
+        (s = D.alloc(&dptrs, sizeof(void*) * chunk)))
       return s;
-    std::vector<cxd> hx;
-    dense_start_block(n, hx);
     std::vector<void*> hp(chunk);
     for (int q = 0; q < chunk; ++q) hp[q] = D.A(q);
-    QBG_CUDA(cudaMemcpyAsync(X0, hx.data(), sizeof(cxd) * hx.size(), cudaMemcpyHostToDevice, st));
     QBG_CUDA(cudaMemcpyAsync(dks, kc.data(), sizeof(cxd) * nk, cudaMemcpyHostToDevice, st));
     QBG_CUDA(cudaMemcpyAsync(dptrs, hp.data(), sizeof(void*) * chunk, cudaMemcpyHostToDevice, st));
-    std::vector<int> info;
-    std::vector<double> hs(chunk);
     for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
       const int c = (int)std::min<int64_t>(chunk, nk - k0);
       D.f.batch = c;
       QBG_TRY(launch_assemble(g->d, dks + k0, c, 0, QBG_PREC_FP64, dptrs, n, st));
       QBG_TRY(lu_factor<double>(D.f, st));
-      QBG_TRY(D.inverse(Cinv));
-      info.assign(c, 0);
-      QBG_CUDA(cudaMemcpyAsync(info.data(), D.f.info, sizeof(int) * c, cudaMemcpyDeviceToHost, st));
-      if (per_cta) {
-        QBG_TRY(sigma_iterate(Cinv, n, c, X0, work, SM_ITERS, 1e-13, dsig, nullptr, nullptr, st));
-        QBG_CUDA(cudaMemcpyAsync(hs.data(), dsig, sizeof(double) * c, cudaMemcpyDeviceToHost, st));
-        QBG_CUDA(cudaStreamSynchronize(st));
-      } else {
-        QBG_CUDA(cudaStreamSynchronize(st));
-        for (int q = 0; q < c; ++q) {
-          hs[q] = 0.0;
-          if (info[q] > 0) continue;
-          cxd* W3 = work;
-          QBG_TRY(sigma_single(Cinv + (size_t)q * n * n, CH, n, X0, W3, W3 + (size_t)n * DENSE_P,
-                               W3 + 2 * (size_t)n * DENSE_P, P, state, SM_ITERS, 1e-13, &hs[q], nullptr, st));
-        }
-      }
-      for (int q = 0; q < c; ++q) sig[k0 + q] = info[q] > 0 ? 0.0 : hs[q];
+      QBG_TRY(sigma_lu(D.f, work, 1e-12, dsig + k0, st));
     }
+    QBG_CUDA(cudaMemcpyAsync(sig, dsig, sizeof(double) * nk, cudaMemcpyDeviceToHost, st));
+    QBG_CUDA(cudaStreamSynchronize(st));
     D.f.batch = chunk;
   }
   return s;

@@ -544,8 +544,8 @@ __global__ void k_pair_rminmax(GeomDev g, unsigned long long* out) {
 // DCT-I coefficients from the values in shared memory with a cosine table the
 // CTA computes once. Bound by FP64 issue. With one thread per panel the
 // (M + 1)^2 cosines of every panel cost twice the Bessel evaluations
-// themselves: 384 nodes of 15600 + 2220 panels of degree 9 took 57 ms that
-// way and 40 ms this way (the whole call 229 -> 212 ms).
+// themselves: eight reduced Beyn disks (384 nodes, 15600 + 2220 panels of
+// degree 9) took 229 ms that way and 212 ms this way.
 constexpr int CHEB_BUILD_THREADS = 128;
 
 __global__ void __launch_bounds__(CHEB_BUILD_THREADS) k_cheb_build(ChebTables t, const cxd* __restrict__ ks) {

@@ -41,6 +41,12 @@ struct Dense64 {
 // batch * 3 * n * DENSE_P elements; vec (optional): n per matrix.
 int sigma_iterate(const cxd* Cinv, int n, int batch, const cxd* X0, cxd* work, int maxit, double tol, double* sig,
                   int* iters, cxd* vec, cudaStream_t st);
+// sigma_min of every A_b of a factored batch (nb = 64, levels = 0) straight from
+// the factors, by Lanczos on (A A^H)^{-1} (see qbg_dense.cu); 0 where info > 0;
+// tol: the Ritz residual relative to the Ritz value; work: batch * sigma_lu_work(n)
+// elements.
+size_t sigma_lu_work(int n);
+int sigma_lu(const LUBatch<double>& f, cxd* work, double tol, double* sig, cudaStream_t st);
 // the fixed n x DENSE_P start block of the iteration (host)
 void dense_start_block(int n, std::vector<cxd>& hx);
 // orthonormal columns of Q (n x p, column-major) in place on the device:
