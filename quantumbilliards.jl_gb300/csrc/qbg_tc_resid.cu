@@ -32,7 +32,7 @@
 // along k 128 B apart, 8-row groups 256 B apart):
 //   T tile (node, 128-row tile mt, ks): planes a = 1..7 of 128 rows (28 KB)
 //   X tile (node, 32-column tile nt, ks): planes b = 1..7 of 64 B' rows (14 KB)
-// One CTA (128 threads) owns 128 rows x 32 complex columns of R: 7 levels x
+// One CTA (512 threads) owns 128 rows x 32 complex columns of R: 7 levels x
 // 64 FP32 TMEM columns. Thread 0 streams the stages through a four-stage
 // ring (full / empty mbarriers, cp.async.bulk) and issues the 28 MMAs of a
 // stage (K = 16 each); every 32 stages (512 real k) it waits for the MMAs and
@@ -69,6 +69,15 @@ struct RLay {
   static constexpr int STAGE = A_TILE + B_TILE;
 };
 constexpr uint32_t RTMEM_COLS = 512;
+// Threads per CTA. The level sums and the epilogue are 2 RBN values a row and
+// ND levels; with one warp per scheduler (128 threads) they took 75 of the 85
+// thousand cycles of a K = 32 product, a third of them waiting for
+// instructions of the fully unrolled code. 16 warps share the rows four ways:
+// warp w reads TMEM lanes 32 (w % 4) .. + 31 and columns RCW (w / 4) .. + RCW - 1
+// of the real and of the imaginary half.
+constexpr int RTHREADS = 512;
+constexpr int RCW = RBN / (RTHREADS / 128);  // complex columns per thread
+static_assert(RCW == 8, "the level reads load eight columns at a time");
 constexpr long long RSPIN = 1ll << 26;
 // D f32, A/B bf16, K-major, N = 64, M = 128
 constexpr uint32_t R_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
@@ -126,6 +135,19 @@ __device__ __forceinline__ void r_bulk(uint32_t dst, const void* src, uint32_t b
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
       "l"(src), "r"(bytes), "r"(mbar)
       : "memory");
+}
+
+// x 2^e, exact: the conversion and the scaling as integer operations on the
+// bit fields (an FP64 instruction costs a warp 64 clocks of its SM quarter
+// here, and the level sums need 2 RBN of them per thread). x is 0 or normal:
+// level sums are multiples of 2^-70.
+__device__ __forceinline__ double scaled_f64(float x, int e) {
+  const uint32_t u = __float_as_uint(x);
+  const int ex = (int)((u >> 23) & 255u);
+  const int E = ex + 896 + e;
+  if (ex == 0) return 0.0;
+  if (E <= 0 || E >= 2047) return ldexp((double)x, e);
+  return __hiloint2double((int)((u & 0x80000000u) | ((uint32_t)E << 20) | ((u & 0x7FFFFFu) >> 3)), (int)(u << 29));
 }
 
 // exact df32 accumulation of one FP32 value
@@ -452,7 +474,7 @@ __global__ void k_a_digits_f64(const cxd* __restrict__ A, long long sA, long lon
 // P: digit planes per operand image (ND <= P); n: rows of T, V and R; ldv:
 // leading dimension of V and R (column l of row i at i + l ldv)
 template <int ND, int P>
-__global__ void __launch_bounds__(128, 1) k_resid_tc(const unsigned char* __restrict__ TD,
+__global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* __restrict__ TD,
                                                      const int* __restrict__ erow,
                                                      const unsigned char* __restrict__ XD,
                                                      const int* __restrict__ fcol, int n, int L, int MT, int NT, int KS,
@@ -495,9 +517,10 @@ __global__ void __launch_bounds__(128, 1) k_resid_tc(const unsigned char* __rest
   const uint32_t tmem = *tmem_slot;
   const uint32_t sbase = r_smem_u32(r_smem);
 
-  float acc_hi[2 * RBN], acc_lo[2 * RBN];
+  const int row = (warp & 3) * 32 + (tid & 31), cw = (warp >> 2) * RCW;  // this thread's row and first column
+  float acc_hi[2 * RCW], acc_lo[2 * RCW];
 #pragma unroll
-  for (int c = 0; c < 2 * RBN; ++c) { acc_hi[c] = 0.f; acc_lo[c] = 0.f; }
+  for (int c = 0; c < 2 * RCW; ++c) { acc_hi[c] = 0.f; acc_lo[c] = 0.f; }
 
   // thread 0: producer and MMA issuer
   const unsigned char* ta = TD + (z * MT + mt) * (long long)KS * RA_TILE;
@@ -568,23 +591,20 @@ __global__ void __launch_bounds__(128, 1) k_resid_tc(const unsigned char* __rest
     const bool flush = (*abort_flag == 0);
     if (flush) {
       __syncwarp();
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
+      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cw;
+#pragma unroll 2
       for (int lev = 0; lev < ND; ++lev) {
-        const float sc = ldexpf(1.f, -7 * (lev + 2));
+        const float sc = __int_as_float((127 - 7 * (lev + 2)) << 23);  // 2^{-7 g}
+        uint32_t v[2 * RCW];
 #pragma unroll
-        for (int qt = 0; qt < 4; ++qt) {
-          uint32_t v[16];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                "=r"(v[15])
-              : "r"(taddr + (uint32_t)(lev * 2 * RBN + qt * 16)));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int h = 0; h < 2; ++h)
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(v[8 * h]), "=r"(v[8 * h + 1]), "=r"(v[8 * h + 2]), "=r"(v[8 * h + 3]), "=r"(v[8 * h + 4]),
+                         "=r"(v[8 * h + 5]), "=r"(v[8 * h + 6]), "=r"(v[8 * h + 7])
+                       : "r"(taddr + (uint32_t)(lev * 2 * RBN + h * RBN)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int c = 0; c < 16; ++c) df_add(acc_hi[qt * 16 + c], acc_lo[qt * 16 + c], __uint_as_float(v[c]) * sc);
-        }
+        for (int c = 0; c < 2 * RCW; ++c) df_add(acc_hi[c], acc_lo[c], __uint_as_float(v[c]) * sc);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -598,16 +618,15 @@ __global__ void __launch_bounds__(128, 1) k_resid_tc(const unsigned char* __rest
     for (int t = freed; t < committed; ++t) r_wait(r_smem_u32(empty + t % RNST), (uint32_t)((t / RNST) & 1));
   }
   if (*abort_flag == 0) {
-    const int i = m0 + tid;
+    const int i = m0 + row;
+    long long lmax = 0;  // bits of the largest |re| + |im| of this row
     if (i < n) {
       const int ei = erow[z * n + i];
       const cxd* Vb = V + z * sV;
       cxd* Rb = R + z * sR;
-      double lmax = 0.0;
-      bool bad = false;
 #pragma unroll
-      for (int c = 0; c < RBN; ++c) {
-        const int col = n0 + c;
+      for (int c = 0; c < RCW; ++c) {
+        const int col = n0 + cw + c;
         if (col >= L) continue;  // full unroll keeps the sums in registers
         const int f = fcol[z * L + col];
         const long long e = (long long)i + (long long)col * ldv;
@@ -616,18 +635,28 @@ __global__ void __launch_bounds__(128, 1) k_resid_tc(const unsigned char* __rest
         if (ei == R_NONFINITE || f == R_NONFINITE) {
           r = cxd(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
         } else {
-          const double re = ldexp((double)acc_hi[c] + (double)acc_lo[c], ei + f);
-          const double im = ldexp((double)acc_hi[RBN + c] + (double)acc_lo[RBN + c], ei + f);
+          // hi + lo is exact in FP64: two FP64 additions per real value
+          const double re = scaled_f64(acc_hi[c], ei + f) + scaled_f64(acc_lo[c], ei + f);
+          const double im = scaled_f64(acc_hi[RCW + c], ei + f) + scaled_f64(acc_lo[RCW + c], ei + f);
           r = cxd(v.re - re, v.im - im);
         }
         Rb[e] = r;
-        const double a = fabs(r.re) + fabs(r.im);
-        bad |= !(a == a);
-        lmax = fmax(lmax, a);
+        if (rmax) {
+          // non-negative doubles order like their bits; a NaN is above +Inf
+          const long long a = __double_as_longlong(fabs(r.re) + fabs(r.im)) & 0x7FFFFFFFFFFFFFFFll;
+          lmax = a > lmax ? a : lmax;
+        }
       }
-      // a NaN (bit pattern above +Inf) wins the unsigned maximum
-      if (rmax)
-        atomicMax(rmax, bad ? 0x7FF8000000000000ull : (unsigned long long)__double_as_longlong(lmax));
+    }
+    if (rmax) {
+      __syncwarp();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const long long a = __shfl_xor_sync(0xffffffffu, lmax, o);
+        lmax = a > lmax ? a : lmax;
+      }
+      if ((tid & 31) == 0)
+        atomicMax(rmax, lmax > 0x7FF0000000000000ll ? 0x7FF8000000000000ull : (unsigned long long)lmax);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -711,11 +740,11 @@ int tc_residual(const TcResidT& t, const cxd* X, long long sX, const cxd* V, lon
   k_x_digits<RD><<<dim3((n + 255) / 256, Lp, c), 256, 0, st>>>(X, sX, n, n, L, NT, t.KS, fcol, XD);
   QBG_LAUNCH_CHECK("k_x_digits");
   if (ndig == 6)
-    k_resid_tc<6, RD><<<dim3(NT, t.MT, c), 128, r_smem_bytes(), st>>>(
+    k_resid_tc<6, RD><<<dim3(NT, t.MT, c), RTHREADS, r_smem_bytes(), st>>>(
         static_cast<const unsigned char*>(t.TD), t.erow, XD, fcol, n, L, t.MT, NT, t.KS, V, sV, R, sR, n,
         reinterpret_cast<unsigned long long*>(rmax), derr);
   else
-    k_resid_tc<RD, RD><<<dim3(NT, t.MT, c), 128, r_smem_bytes(), st>>>(
+    k_resid_tc<RD, RD><<<dim3(NT, t.MT, c), RTHREADS, r_smem_bytes(), st>>>(
         static_cast<const unsigned char*>(t.TD), t.erow, XD, fcol, n, L, t.MT, NT, t.KS, V, sV, R, sR, n,
         reinterpret_cast<unsigned long long*>(rmax), derr);
   QBG_LAUNCH_CHECK("k_resid_tc");
@@ -790,7 +819,7 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
     launched("k_x_digits");
   }
   if (!s) {
-    k_resid_tc<P, P><<<dim3(NT, MT, batch), 128, r_smem_bytes<P>(), st>>>(TDm, erow, XDm, fcol, M, N, MT, NT, KS,
+    k_resid_tc<P, P><<<dim3(NT, MT, batch), RTHREADS, r_smem_bytes<P>(), st>>>(TDm, erow, XDm, fcol, M, N, MT, NT, KS,
                                                                            C, sC, C, sC, ldc, nullptr, derr);
     launched("k_resid_tc");
   }
