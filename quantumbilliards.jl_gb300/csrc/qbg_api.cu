@@ -461,7 +461,7 @@ qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig)
       QBG_TRY(sigma_lu(D.f, work, 1e-12, dsig + k0, st));
     }
     QBG_CUDA(cudaMemcpyAsync(sig, dsig, sizeof(double) * nk, cudaMemcpyDeviceToHost, st));
-    QBG_CUDA(cudaStreamSynchronize(st));
+    QBG_TRY(tc_check(st));  // waits for the stream
     D.f.batch = chunk;
   }
   return s;

@@ -250,7 +250,7 @@ int load(qbg_beyn* b, int n0, int c) {
   std::vector<int> hinfo(c);
   QBG_CUDA(cudaMemcpyAsync(hinfo.data(), info, sizeof(int) * c, cudaMemcpyDeviceToHost, st));
   QBG_CUDA(cudaStreamSynchronize(st));
-  if (b->prec != QBG_PREC_FP64) QBG_TRY(tc_check(st));
+  QBG_TRY(tc_check(st));
   for (int v : hinfo) b->singular += (v != 0);
   float ma = 0.f, mf = 0.f;
   QBG_CUDA(cudaEventElapsedTime(&ma, b->ev[0], b->ev[1]));
@@ -654,7 +654,7 @@ int moments_impl(qbg_beyn* b, const double* V, int64_t L, double* A0, double* A1
   cudaEventElapsedTime(&ms_total, b->ev[3], e_end);
   cudaEventDestroy(e_end);
   if (e != cudaSuccess) return cuda_status(e, "qbg_beyn_moments");
-  if (b->prec != QBG_PREC_FP64) QBG_TRY(tc_check(st));
+  QBG_TRY(tc_check(st));
   double ms_solves = 0.0;
   for (size_t q = 0; q + 1 < c.sev.size(); q += 2) {
     float ms = 0.f;

@@ -990,15 +990,77 @@ static std::atomic<int> g_f64_tc{[] {
   return (e && *e) ? (std::atoi(e) != 0 ? 1 : 0) : 1;
 }()};
 
+// A 64 x 64 FP64 tile takes one SM K x 4.3 us whatever part of it the product
+// fills (2 FMAs per clock), the three launches of the tensor-core product about
+// 25 us: from K = 16 on the tensor cores are the faster side down to the
+// smallest products. (24 operators of n = 1502: 32-row products left on the FP64
+// pipe took 53 of 134 ms.)
+static bool f64_tc(int M, int N, int K, int batch) {
+  return g_f64_tc.load() && M >= 16 && N >= 16 && K >= 16 && batch <= 65535;
+}
+
 template <class T>
 static int gemm_sub(int M, int N, int K, const cx<T>* A, long long lda, long long sA, const cx<T>* B, long long ldb,
                     long long sB, cx<T>* C, long long ldc, long long sC, int batch, cudaStream_t st) {
   if constexpr (sizeof(T) == 8) {
-    if (g_f64_tc.load() && M >= 256 && N >= 64 && K >= 16 && batch <= 65535)
+    if (f64_tc(M, N, K, batch))
       return tc_gemm_sub_f64(M, N, K, reinterpret_cast<const cxd*>(A), lda, sA, reinterpret_cast<const cxd*>(B), ldb,
                              sB, reinterpret_cast<cxd*>(C), ldc, sC, batch, st);
   }
   return gemm_batched<T>(M, N, K, cx<T>(-1, 0), A, lda, sA, B, ldb, sB, cx<T>(1, 0), C, ldc, sC, batch, st);
+}
+
+// X = A X in place for w x w blocks A (leading dimension W), every product in
+// FP64: the diagonal-block steps of the triangular solves. (Through digits they
+// doubled the rounding error of the solutions, 1.4e-13 -> 2.0e-13 on a 1502-node
+// Beyn disk: the rows of an inverse of U vary too much for one scale per row.
+// The U rows of the factorisation showed no such loss.) One output per thread,
+// 256 / W columns per CTA, so that a few right-hand sides still reach every SM:
+// 32 x 64 outputs of 24 operators on the 64 x 64 GEMM tile kept 24 SMs busy.
+template <int W>
+__global__ void __launch_bounds__(256) k_block_mul_f64(const cxd* __restrict__ A, long long sA, int w, cxd* X,
+                                                       long long ldx, long long sX, int N) {
+  constexpr int NC = 256 / W;
+  __shared__ cxd xs[NC][W];
+  const int i = threadIdx.x % W, c = threadIdx.x / W, col = blockIdx.x * NC + c;
+  const cxd* a = A + blockIdx.y * sA + i;
+  cxd* x = X + blockIdx.y * sX + (long long)col * ldx;
+  const bool in = i < w && col < N;
+  xs[c][i] = in ? x[i] : cxd(0.0, 0.0);
+  __syncthreads();
+  if (!in) return;
+  cxd acc(0.0, 0.0);
+#pragma unroll 8
+  for (int k = 0; k < w; ++k) cfma(acc, a[(long long)k * W], xs[c][k]);
+  x[i] = acc;
+}
+
+template <class T>
+static int solve_block_mul(int w, int N, const cx<T>* A, int nb, long long sA, cx<T>* X, long long ldx, long long sX,
+                           int batch, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    if (batch <= 65535 && (nb == 32 || nb == 64)) {
+      if (nb == 32)
+        k_block_mul_f64<32><<<dim3((N + 7) / 8, batch), 256, 0, st>>>(A, sA, w, X, ldx, sX, N);
+      else
+        k_block_mul_f64<64><<<dim3((N + 3) / 4, batch), 256, 0, st>>>(A, sA, w, X, ldx, sX, N);
+      QBG_LAUNCH_CHECK("k_block_mul_f64");
+      return QBG_OK;
+    }
+  }
+  return gemm_batched<T>(w, N, w, cx<T>(1, 0), A, nb, sA, X, ldx, sX, cx<T>(0, 0), X, ldx, sX, batch, st);
+}
+
+// X = A X in place for w x w blocks A: the U rows of the factorisation
+template <class T>
+static int block_mul(int w, int N, const cx<T>* A, long long lda, long long sA, cx<T>* X, long long ldx, long long sX,
+                     int batch, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    if (f64_tc(w, N, w, batch))
+      return tc_block_mul_f64(w, N, reinterpret_cast<const cxd*>(A), lda, sA, reinterpret_cast<cxd*>(X), ldx, sX, batch,
+                              st);
+  }
+  return gemm_batched<T>(w, N, w, cx<T>(1, 0), A, lda, sA, X, ldx, sX, cx<T>(0, 0), X, ldx, sX, batch, st);
 }
 
 template <class T>
@@ -1071,7 +1133,6 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   // so the factors are those of the one-level algorithm.
   // panels per outer block: set_lu_plan (or QBG_LU_OUTER in the environment), 1..16, default 4
   const int LU_OUTER = g_lu_outer.load();
-  const cx<T> one(1, 0), mone(-1, 0), zero(0, 0);
   auto linv = [&](int j) { return f.Linv + (long long)(j / nb) * nb * nb; };
   const long long sLinv = (long long)f.nblk * nb * nb;
   for (int J0 = 0; J0 < n; J0 += LU_OUTER * nb) {
@@ -1105,8 +1166,7 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
       const int rin = E - j0 - w;  // columns of this outer block right of the panel
       if (rin > 0) {
         // U12 = inv(L11) A12 and A22 -= L21 U12 on the outer block's columns
-        int s = gemm_batched<T>(w, rin, w, one, linv(j0), nb, sLinv, f.A + j0 + (long long)(j0 + w) * n, n,
-                                f.stride, zero, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, st);
+        int s = block_mul<T>(w, rin, linv(j0), nb, sLinv, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, st);
         if (s) return s;
         s = gemm_sub<T>(n - j0 - w, rin, w, f.A + (j0 + w) + (long long)j0 * n, n, f.stride,
                         f.A + j0 + (long long)(j0 + w) * n, n, f.stride, f.A + (j0 + w) + (long long)(j0 + w) * n, n,
@@ -1119,8 +1179,7 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
       // U rows of the outer block on the trailing columns: U_b = inv(L_bb) (A_b - sum_{b'<b} L_bb' U_b')
       for (int j0 = J0; j0 < E; j0 += nb) {
         const int w = min(nb, E - j0);
-        int s = gemm_batched<T>(w, rest, w, one, linv(j0), nb, sLinv, f.A + j0 + (long long)E * n, n, f.stride,
-                                zero, f.A + j0 + (long long)E * n, n, f.stride, batch, st);
+        int s = block_mul<T>(w, rest, linv(j0), nb, sLinv, f.A + j0 + (long long)E * n, n, f.stride, batch, st);
         if (s) return s;
         const int below = E - j0 - w;
         if (below > 0) {
@@ -1269,8 +1328,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
   const long long sInv = (long long)f.nblk * nb * nb;
   for (int blk = 0; blk < f.nblk; ++blk) {
     const int r0 = blk * nb, w = min(nb, n - r0);
-    int s = gemm_batched<T>(w, L, w, cx<T>(1, 0), f.Linv + (long long)blk * nb * nb, nb, sInv, X + r0, n, sX,
-                            cx<T>(0, 0), X + r0, n, sX, batch, st);
+    int s = solve_block_mul<T>(w, L, f.Linv + (long long)blk * nb * nb, nb, sInv, X + r0, n, sX, batch, st);
     if (s) return s;
     const int rest = n - r0 - w;
     if (rest > 0) {
@@ -1281,8 +1339,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
   }
   for (int blk = f.nblk - 1; blk >= 0; --blk) {
     const int r0 = blk * nb, w = min(nb, n - r0);
-    int s = gemm_batched<T>(w, L, w, cx<T>(1, 0), f.Uinv + (long long)blk * nb * nb, nb, sInv, X + r0, n, sX,
-                            cx<T>(0, 0), X + r0, n, sX, batch, st);
+    int s = solve_block_mul<T>(w, L, f.Uinv + (long long)blk * nb * nb, nb, sInv, X + r0, n, sX, batch, st);
     if (s) return s;
     if (r0 > 0) {
       s = gemm_sub<T>(r0, L, w, f.A + (long long)r0 * n, n, f.stride, X + r0, n, sX, X, n, sX, batch, st);

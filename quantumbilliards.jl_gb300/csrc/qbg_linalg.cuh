@@ -144,6 +144,10 @@ int tc_residual(const TcResidT& t, const cxd* X, long long sX, const cxd* V, lon
 // (qbg_tc_resid.cu); scratch from the pool, stream-ordered
 int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long sA, const cxd* B, long long ldb,
                     long long sB, cxd* C, long long ldc, long long sC, int batch, cudaStream_t st);
+// X_b = A_b X_b in place for w x w blocks A_b, w <= 128: the diagonal of A in
+// FP64, the rest as above
+int tc_block_mul_f64(int w, int N, const cxd* A, long long lda, long long sA, cxd* X, long long ldx, long long sX,
+                     int batch, cudaStream_t st);
 // device address of the tensor-core error flag (shared by the GEMM and the residual)
 int tc_error_ptr(int** p);
 

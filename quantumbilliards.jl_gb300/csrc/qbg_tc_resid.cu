@@ -15,8 +15,8 @@
 // a + b = g <= 8 (28 pairs, 7 levels g = 2..8) are summed per level in its
 // own TMEM accumulator. A level collects at most 7 pairs, so over 512 real
 // terms its partial sum stays below 7 * 2^21 < 2^24 and is exact; every 512
-// terms the levels are read back and added, scaled by 2^{-7g}, into
-// double-float (hi + lo FP32) sums, which carry ~48 bits. (A residual for a
+// terms the levels are read back and added, as integers, into two 64-bit sums
+// of levels each, which are rounded to FP64 once at the end. (A residual for a
 // refinement sweep that is not the last may use the leading six digits of
 // both operands: 21 pairs in 6 levels, ~2^-40 of the scales.) The pairs left out
 // (a + b >= 9) and the truncation of both digit expansions are below 2^-47 of
@@ -36,7 +36,7 @@
 // 64 FP32 TMEM columns. Thread 0 streams the stages through a four-stage
 // ring (full / empty mbarriers, cp.async.bulk) and issues the 28 MMAs of a
 // stage (K = 16 each); every 32 stages (512 real k) it waits for the MMAs and
-// all threads add the level sums into their double-float accumulators. Every
+// all threads add the level sums into their integer accumulators. Every
 // wait is bounded (1e9 SM cycles): on a timeout the CTA records an error,
 // waits (bounded) for the copies and MMAs it started, frees its TMEM and
 // returns without writing R.
@@ -137,28 +137,37 @@ __device__ __forceinline__ void r_bulk(uint32_t dst, const void* src, uint32_t b
       : "memory");
 }
 
-// x 2^e, exact: the conversion and the scaling as integer operations on the
-// bit fields (an FP64 instruction costs a warp 64 clocks of its SM quarter
-// here, and the level sums need 2 RBN of them per thread). x is 0 or normal:
-// level sums are multiples of 2^-70.
-__device__ __forceinline__ double scaled_f64(float x, int e) {
-  const uint32_t u = __float_as_uint(x);
-  const int ex = (int)((u >> 23) & 255u);
-  const int E = ex + 896 + e;
-  if (ex == 0) return 0.0;
-  if (E <= 0 || E >= 2047) return ldexp((double)x, e);
-  return __hiloint2double((int)((u & 0x80000000u) | ((uint32_t)E << 20) | ((u & 0x7FFFFFu) >> 3)), (int)(u << 29));
-}
-
-// exact df32 accumulation of one FP32 value
-__device__ __forceinline__ void df_add(float& hi, float& lo, float x) {
-  const float s = hi + x;
-  const float bb = s - hi;
-  const float e = (hi - (s - bb)) + (x - bb);
-  lo += e;
-  const float h2 = s + lo;
-  lo -= h2 - s;
-  hi = h2;
+// (hi 2^SH + lo) 2^e rounded to FP64 (to nearest even), as integer operations:
+// an FP64 instruction costs a warp 64 clocks of its SM quarter here
+template <int SH>
+__device__ __forceinline__ double fixed_to_f64(long long hi, long long lo, int e) {
+  const __int128 t = ((__int128)hi << SH) + lo;
+  const bool neg = t < 0;
+  const unsigned __int128 u = neg ? -(unsigned __int128)t : (unsigned __int128)t;
+  unsigned long long h = (unsigned long long)(u >> 64), l = (unsigned long long)u, m;
+  int top;  // position of the leading bit
+  bool sticky = false;
+  if (h) {
+    const int s = __clzll((long long)h);
+    m = s ? (h << s) | (l >> (64 - s)) : h;
+    sticky = (l << s) != 0;
+    top = 127 - s;
+  } else {
+    if (!l) return 0.0;
+    const int s = __clzll((long long)l);
+    m = l << s;
+    top = 63 - s;
+  }
+  unsigned long long keep = m >> 11;
+  const unsigned int rem = (unsigned int)m & 0x7FFu;
+  keep += (rem > 0x400u || (rem == 0x400u && (sticky || (keep & 1ull)))) ? 1ull : 0ull;
+  const int E = top + 1023 + e;
+  if (E <= 0 || E >= 2046) {
+    const double v = ldexp((double)keep, top - 52 + e);
+    return neg ? -v : v;
+  }
+  const unsigned long long bits = ((unsigned long long)(E - 1) << 52) + keep;
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
 }  // namespace
@@ -465,6 +474,142 @@ __global__ void k_a_digits_f64(const cxd* __restrict__ A, long long sA, long lon
   }
 }
 
+// Exponents and digits of both operands of a product with K <= PREP_K in one
+// pass each: a CTA holds 32 whole rows of A in shared memory, a warp one whole
+// column of B in registers, so each value is read once and a product is three
+// launches. The maxima are integer comparisons of the bit fields. k in
+// [K, 8 ceil(K / 8)) is written as zero; image rows past M and columns past N
+// are left as they are: they reach no stored row or column of the product.
+constexpr int PREP_K = 128;
+
+// exponent e with |v| < 2^(e - 1) from the largest magnitude's bits
+__device__ __forceinline__ int exp_of_bits(long long m) {
+  if (m >= 0x7FF0000000000000ll) return R_NONFINITE;
+  const int ex = (int)(m >> 52);
+  if (ex) return ex - 1021;
+  if (m == 0) return 0;
+  int E = 0;
+  frexp(__longlong_as_double(m), &E);
+  return E + 1;
+}
+__device__ __forceinline__ long long mag_bits(cxd v) {
+  const long long a = __double_as_longlong(v.re) & 0x7FFFFFFFFFFFFFFFll;
+  const long long b = __double_as_longlong(v.im) & 0x7FFFFFFFFFFFFFFFll;
+  return a > b ? a : b;
+}
+
+// grid (ceil(M / 32), batch), block (32, 8), dynamic smem ceil8(K) * 33 cxd;
+// offdiag: the diagonal entries count as zero
+template <int P>
+__global__ void __launch_bounds__(256) k_a_prep_f64(const cxd* __restrict__ A, long long sA, long long lda, int M, int K,
+                                                    int MT, int KS, int* __restrict__ erow,
+                                                    unsigned char* __restrict__ TD, int offdiag) {
+  extern __shared__ __align__(16) unsigned char p_smem[];
+  cxd* tv = reinterpret_cast<cxd*>(p_smem);  // [k][33]
+  __shared__ long long red[8][33];
+  __shared__ int es[32];
+  const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 32 + tx;
+  const int i0 = blockIdx.x * 32, Kp = (K + 7) & ~7;
+  const long long b = blockIdx.y;
+  const cxd* a = A + b * sA;
+  long long m = 0;
+  for (int k = ty; k < Kp; k += 8) {
+    const bool in = i0 + tx < M && k < K && !(offdiag && i0 + tx == k);
+    const cxd v = in ? a[(long long)(i0 + tx) + (long long)k * lda] : cxd(0.0, 0.0);
+    tv[k * 33 + tx] = v;
+    const long long q = mag_bits(v);
+    m = q > m ? q : m;
+  }
+  red[ty][tx] = m;
+  __syncthreads();
+  if (ty == 0) {
+#pragma unroll
+    for (int r = 1; r < 8; ++r) m = red[r][tx] > m ? red[r][tx] : m;
+    const int e = exp_of_bits(m);
+    es[tx] = e;
+    if (i0 + tx < M) erow[b * M + i0 + tx] = e;
+  }
+  __syncthreads();
+  for (int w = t; w < 32 * Kp; w += 256) {
+    const int e4 = w & 3, rr = (w >> 2) & 7, rg = (w >> 5) & 3, cs = w >> 7;  // cs: (stage, core column)
+    const int il = rg * 8 + rr, k = (cs >> 1) * 8 + (cs & 1) * 4 + e4, i = i0 + il;
+    if (i >= M) continue;
+    const cxd v = tv[k * 33 + il];
+    const int e = es[il];
+    float dr[P], di[P];
+    if (e == R_NONFINITE) {
+#pragma unroll
+      for (int q = 0; q < P; ++q) { dr[q] = 0.f; di[q] = 0.f; }
+    } else {
+      digitsP<P>(fx_f64(v.re, 7 * P - e), dr);
+      digitsP<P>(fx_f64(v.im, 7 * P - e), di);
+    }
+    unsigned char* tile =
+        TD + ((b * MT + (i >> 7)) * (long long)KS + (k >> 3)) * RLay<P>::A_TILE + img_off(i & 127, (2 * k) & 15);
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      __nv_bfloat162 pq;
+      pq.x = __float2bfloat16_rn(dr[q]);
+      pq.y = __float2bfloat16_rn(di[q]);
+      *reinterpret_cast<__nv_bfloat162*>(tile + q * RA_PLANE) = pq;
+    }
+  }
+}
+
+// grid (ceil(N / 8), batch), block 256: one warp per column
+template <int P>
+__global__ void __launch_bounds__(256) k_x_prep_f64(const cxd* __restrict__ X, long long sX, long long ldx, int K, int N,
+                                                    int NT, int KS, int* __restrict__ fcol,
+                                                    unsigned char* __restrict__ XD) {
+  const int lane = threadIdx.x & 31, l = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long b = blockIdx.y;
+  if (l >= N) return;
+  const int Kp = (K + 7) & ~7;
+  const cxd* x = X + b * sX + (long long)l * ldx;
+  cxd v[PREP_K / 32];
+  long long m = 0;
+#pragma unroll
+  for (int q = 0; q < PREP_K / 32; ++q) {
+    const int k = lane + 32 * q;
+    v[q] = k < K ? x[k] : cxd(0.0, 0.0);
+    const long long a = mag_bits(v[q]);
+    m = a > m ? a : m;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long a = __shfl_xor_sync(0xffffffffu, m, o);
+    m = a > m ? a : m;
+  }
+  const int f = exp_of_bits(m);
+  if (lane == 0) fcol[b * N + l] = f;
+  const int j = l & (RBN - 1);
+#pragma unroll
+  for (int q = 0; q < PREP_K / 32; ++q) {
+    const int k = lane + 32 * q;
+    if (k >= Kp) break;
+    float dr[P], di[P];
+    if (f == R_NONFINITE) {
+#pragma unroll
+      for (int c = 0; c < P; ++c) { dr[c] = 0.f; di[c] = 0.f; }
+    } else {
+      digitsP<P>(fx_f64(v[q].re, 7 * P - f), dr);
+      digitsP<P>(fx_f64(v[q].im, 7 * P - f), di);
+    }
+    unsigned char* tile = XD + ((b * NT + (l / RBN)) * (long long)KS + (k >> 3)) * RLay<P>::B_TILE;
+    const uint32_t o_re = img_off(j, (2 * k) & 15), o_im = img_off(RBN + j, (2 * k) & 15);
+#pragma unroll
+    for (int c = 0; c < P; ++c) {
+      __nv_bfloat162 pr, pi;
+      pr.x = __float2bfloat16_rn(dr[c]);
+      pr.y = __float2bfloat16_rn(-di[c]);
+      pi.x = __float2bfloat16_rn(di[c]);
+      pi.y = __float2bfloat16_rn(dr[c]);
+      *reinterpret_cast<__nv_bfloat162*>(tile + c * RB_PLANE + o_re) = pr;
+      *reinterpret_cast<__nv_bfloat162*>(tile + c * RB_PLANE + o_im) = pi;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // R = V - T X from the digit planes; grid (Lp / 32, ceil(n / 128), batch)
 // ---------------------------------------------------------------------------
@@ -472,14 +617,17 @@ __global__ void k_a_digits_f64(const cxd* __restrict__ A, long long sA, long lon
 // ND = RD is the full product, a smaller ND a residual to ~2^-(7 ND) of the
 // scales (for refinement sweeps whose correction is not the last)
 // P: digit planes per operand image (ND <= P); n: rows of T, V and R; ldv:
-// leading dimension of V and R (column l of row i at i + l ldv)
+// leading dimension of V and R (column l of row i at i + l ldv); Dg (optional,
+// the diagonal entries Dg[i ldd] of row i): R = diag(Dg) V + T X
 template <int ND, int P>
 __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* __restrict__ TD,
                                                      const int* __restrict__ erow,
                                                      const unsigned char* __restrict__ XD,
                                                      const int* __restrict__ fcol, int n, int L, int MT, int NT, int KS,
-                                                     const cxd* __restrict__ V, long long sV, cxd* R, long long sR,
-                                                     long long ldv, unsigned long long* rmax, int* err) {
+                                                     const cxd* V, long long sV, cxd* R, long long sR, long long ldv,
+                                                     unsigned long long* rmax, int* err,
+                                                     const cxd* __restrict__ Dg = nullptr, long long sD = 0,
+                                                     long long ldd = 0) {
   constexpr int RA_TILE = RLay<P>::A_TILE, RB_TILE = RLay<P>::B_TILE, RSTAGE = RLay<P>::STAGE;
   // stages between exact flushes: a level of ND digits collects up to ND
   // pairs, so 16 stages (256 real k) keep eight-digit level sums below 2^23
@@ -518,9 +666,11 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
   const uint32_t sbase = r_smem_u32(r_smem);
 
   const int row = (warp & 3) * 32 + (tid & 31), cw = (warp >> 2) * RCW;  // this thread's row and first column
-  float acc_hi[2 * RCW], acc_lo[2 * RCW];
+  // the sums of levels 2 .. 5 in units of 2^-35 and of levels 6 .. ND + 1 in
+  // units of 2^{-7 (ND + 1)}, exact
+  long long acc_hi[2 * RCW], acc_lo[2 * RCW];
 #pragma unroll
-  for (int c = 0; c < 2 * RCW; ++c) { acc_hi[c] = 0.f; acc_lo[c] = 0.f; }
+  for (int c = 0; c < 2 * RCW; ++c) { acc_hi[c] = 0; acc_lo[c] = 0; }
 
   // thread 0: producer and MMA issuer
   const unsigned char* ta = TD + (z * MT + mt) * (long long)KS * RA_TILE;
@@ -592,19 +742,34 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
     if (flush) {
       __syncwarp();
       const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cw;
-#pragma unroll 2
-      for (int lev = 0; lev < ND; ++lev) {
-        const float sc = __int_as_float((127 - 7 * (lev + 2)) << 23);  // 2^{-7 g}
-        uint32_t v[2 * RCW];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h) {  // the real columns, then the imaginary ones
+        auto level = [&](int lev, uint32_t (&v)[RCW]) {
           asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                       : "=r"(v[8 * h]), "=r"(v[8 * h + 1]), "=r"(v[8 * h + 2]), "=r"(v[8 * h + 3]), "=r"(v[8 * h + 4]),
-                         "=r"(v[8 * h + 5]), "=r"(v[8 * h + 6]), "=r"(v[8 * h + 7])
+                       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                        : "r"(taddr + (uint32_t)(lev * 2 * RBN + h * RBN)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        };
+        // two neighbouring levels S_g 128 + S_{g+1} stay below 2^31: S_g counts
+        // at most g - 1 <= 6 pairs where another level follows, 2^21 each
 #pragma unroll
-        for (int c = 0; c < 2 * RCW; ++c) df_add(acc_hi[c], acc_lo[c], __uint_as_float(v[c]) * sc);
+        for (int half = 0; half < 2; ++half) {
+          const int l0 = half ? 4 : 0, cnt = half ? ND - 4 : 4;
+          uint32_t v[4][RCW];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q < cnt) level(l0 + q, v[q]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < RCW; ++c) {
+            int p = __float2int_rn(__uint_as_float(v[0][c])), q = 0;
+            if (cnt > 1) p = p * 128 + __float2int_rn(__uint_as_float(v[1][c]));
+            if (cnt > 2) q = __float2int_rn(__uint_as_float(v[2][c]));
+            if (cnt > 3) q = q * 128 + __float2int_rn(__uint_as_float(v[3][c]));
+            const long long t = cnt > 3 ? (long long)p * 16384 + q : (cnt > 2 ? (long long)p * 128 + q : (long long)p);
+            if (half) acc_lo[h * RCW + c] += t;
+            else acc_hi[h * RCW + c] += t;
+          }
+        }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -624,6 +789,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
       const int ei = erow[z * n + i];
       const cxd* Vb = V + z * sV;
       cxd* Rb = R + z * sR;
+      const cxd dg = Dg ? Dg[z * sD + (long long)i * ldd] : cxd(0.0, 0.0);
 #pragma unroll
       for (int c = 0; c < RCW; ++c) {
         const int col = n0 + cw + c;
@@ -635,10 +801,15 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
         if (ei == R_NONFINITE || f == R_NONFINITE) {
           r = cxd(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
         } else {
-          // hi + lo is exact in FP64: two FP64 additions per real value
-          const double re = scaled_f64(acc_hi[c], ei + f) + scaled_f64(acc_lo[c], ei + f);
-          const double im = scaled_f64(acc_hi[RCW + c], ei + f) + scaled_f64(acc_lo[RCW + c], ei + f);
-          r = cxd(v.re - re, v.im - im);
+          const int e2 = ei + f - 7 * (ND + 1);
+          const double re = fixed_to_f64<7 * (ND - 4)>(acc_hi[c], acc_lo[c], e2);
+          const double im = fixed_to_f64<7 * (ND - 4)>(acc_hi[RCW + c], acc_lo[RCW + c], e2);
+          if (Dg) {
+            r = cxd(re, im);
+            cfma(r, dg, v);
+          } else {
+            r = cxd(v.re - re, v.im - im);
+          }
         }
         Rb[e] = r;
         if (rmax) {
@@ -756,13 +927,19 @@ int tc_residual(const TcResidT& t, const cxd* X, long long sX, const cxd* V, lon
 // operands are cut into eight balanced 7-bit digits against the row maxima of
 // A and the column maxima of B (56-bit fixed point), the 36 digit pairs with
 // a + b <= 9 are multiplied exactly on the tensor cores into 8 TMEM level
-// sums (exact FP32 integers over 256 real k), the levels are added in
-// double-float and subtracted from C in FP64: per product term the error is
+// sums (exact FP32 integers over 256 real k), the levels are added exactly,
+// rounded to FP64 and subtracted from C: per product term the error is
 // ~2^-56 of max_k |A_ik| max_k |B_kj|, the order of an FP64 GEMM's rounding.
-int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long sA, const cxd* B, long long ldb,
-                    long long sB, cxd* C, long long ldc, long long sC, int batch, cudaStream_t st) {
+// diag (M = K <= PREP_K, C = B): C_b = A_b B_b in place, with A's diagonal
+// applied in FP64 and only the rest from digits, so that the digits' scale is
+// that of the off-diagonal entries (the triangular inverses of the LU, whose
+// diagonal dominates their rows). The digits of both operands are taken before
+// C is written, so C may overlap A or B.
+static int tc_gemm_f64(int M, int N, int K, const cxd* A, long long lda, long long sA, const cxd* B, long long ldb,
+                       long long sB, cxd* C, long long ldc, long long sC, int batch, cudaStream_t st, bool diag) {
   constexpr int P = 8;
-  if (M < 1 || N < 1 || K < 1 || batch < 1 || batch > 65535 || lda < M || ldb < K || ldc < M) {
+  if (M < 1 || N < 1 || K < 1 || batch < 1 || batch > 65535 || lda < M || ldb < K || ldc < M ||
+      (diag && (M != K || K > PREP_K || C != B || ldc != ldb || sC != sB))) {
     set_error("tc_gemm_sub_f64: bad sizes");
     return QBG_EINVAL;
   }
@@ -780,6 +957,8 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
   if (dev >= 0 && dev < 64 && !attr[dev]) {
     QBG_CUDA(cudaFuncSetAttribute(k_resid_tc<P, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)r_smem_bytes<P>()));
+    QBG_CUDA(cudaFuncSetAttribute(k_a_prep_f64<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  PREP_K * 33 * (int)sizeof(cxd)));
     attr[dev] = true;
   }
   unsigned char* mem = nullptr;
@@ -789,12 +968,13 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
   int* erow = reinterpret_cast<int*>(mem + td_r + xd_r);
   int* fcol = reinterpret_cast<int*>(mem + td_r + xd_r + er);
   int s = QBG_OK;
+  const bool prep = K <= PREP_K;
   // images of rows past M, k past K or columns past N stay zero
-  if (M % RBM || K % 8) {
+  if (!prep && (M % RBM || K % 8)) {
     cudaError_t e = cudaMemsetAsync(TDm, 0, td, st);
     if (e != cudaSuccess) s = cuda_status(e, "tc_gemm_sub_f64 memset");
   }
-  if (!s && (K % 8 || N % RBN)) {
+  if (!prep && !s && (K % 8 || N % RBN)) {
     cudaError_t e = cudaMemsetAsync(XDm, 0, xd, st);
     if (e != cudaSuccess) s = cuda_status(e, "tc_gemm_sub_f64 memset");
   }
@@ -804,7 +984,16 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
     if (e != cudaSuccess) s = cuda_status(e, what);
     return s == QBG_OK;
   };
-  if (!s) {
+  if (prep) {
+    const size_t sm = (size_t)((K + 7) & ~7) * 33 * sizeof(cxd);
+    k_a_prep_f64<P><<<dim3((M + 31) / 32, batch), dim3(32, 8), sm, st>>>(A, sA, lda, M, K, MT, KS, erow, TDm,
+                                                                                   diag ? 1 : 0);
+    if (launched("k_a_prep_f64")) {
+      k_x_prep_f64<P><<<dim3((N + 7) / 8, batch), 256, 0, st>>>(B, sB, ldb, K, N, NT, KS, fcol, XDm);
+      launched("k_x_prep_f64");
+    }
+  }
+  if (!prep && !s) {
     k_a_rowexp_f64<<<dim3((M + 31) / 32, batch), dim3(32, 8), 0, st>>>(A, sA, lda, M, K, erow);
     if (launched("k_a_rowexp_f64")) {
       k_a_digits_f64<P><<<dim3((M + 31) / 32, (K + 31) / 32, batch), dim3(32, 8), 0, st>>>(A, sA, lda, M, K, MT, KS,
@@ -812,7 +1001,7 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
       launched("k_a_digits_f64");
     }
   }
-  if (!s) {
+  if (!prep && !s) {
     k_x_colexp<<<dim3(N, batch), 256, 0, st>>>(B, sB, ldb, K, N, fcol);
     if (launched("k_x_colexp"))
       k_x_digits<P><<<dim3((K + 255) / 256, Lp, batch), 256, 0, st>>>(B, sB, ldb, K, N, NT, KS, fcol, XDm);
@@ -820,11 +1009,22 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
   }
   if (!s) {
     k_resid_tc<P, P><<<dim3(NT, MT, batch), RTHREADS, r_smem_bytes<P>(), st>>>(TDm, erow, XDm, fcol, M, N, MT, NT, KS,
-                                                                           C, sC, C, sC, ldc, nullptr, derr);
+                                                                           C, sC, C, sC, ldc, nullptr, derr,
+                                                                           diag ? A : nullptr, sA, lda + 1);
     launched("k_resid_tc");
   }
   dfree(mem, st);
   return s;
+}
+
+int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long sA, const cxd* B, long long ldb,
+                    long long sB, cxd* C, long long ldc, long long sC, int batch, cudaStream_t st) {
+  return tc_gemm_f64(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, st, false);
+}
+
+int tc_block_mul_f64(int w, int N, const cxd* A, long long lda, long long sA, cxd* X, long long ldx, long long sX,
+                     int batch, cudaStream_t st) {
+  return tc_gemm_f64(w, N, w, A, lda, sA, X, ldx, sX, X, ldx, sX, batch, st, true);
 }
 
 }  // namespace qbg
