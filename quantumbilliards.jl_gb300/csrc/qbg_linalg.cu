@@ -556,14 +556,15 @@ __global__ void __launch_bounds__(1024) k_getrf_panel_smem(cx<T>* A, int n, long
 // pivot bookkeeping then outweighing the split update.)
 // ---------------------------------------------------------------------------
 constexpr int PC_THREADS = 256;
-// largest rows per CTA: 64 columns within the dynamic shared memory left
-// beside the push buffers, whose static size grows with the cluster: 8 CTAs
-// 432 complex64 / 200 complex128 rows, 16 CTAs 416 / 192 rows
+// largest rows per CTA of a panel of w columns: what the push buffers, whose
+// size grows with the cluster, leave of the 227 KB of shared memory
 template <class T, int CS>
-constexpr int pc_max_rpc() { return sizeof(T) == 4 ? (CS == 8 ? 432 : 416) : (CS == 8 ? 200 : 192); }
+constexpr int pc_max_rpc(int w) {
+  return (227 * 1024 - 2048 - (2 * CS + 2) * 64 * (int)sizeof(cx<T>)) / (w * (int)sizeof(cx<T>));
+}
 
-// CS = 8 (portable cluster size) or 16 (non-portable, for panels too tall for
-// 8 CTAs' shared memory, used when the device can hold such a cluster)
+// CS = 2, 4, 8 (portable cluster sizes) or 16 (non-portable, used when the
+// device can hold such a cluster)
 template <class T, int CS>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(PC_THREADS)
     k_getrf_panel_cluster(cx<T>* A, int n, long long stride, int j0, int nb, int rpc, int* ipiv, int* info) {
@@ -1063,6 +1064,83 @@ static int block_mul(int w, int N, const cx<T>* A, long long lda, long long sA, 
   return gemm_batched<T>(w, N, w, cx<T>(1, 0), A, lda, sA, X, ldx, sX, cx<T>(0, 0), X, ldx, sX, batch, st);
 }
 
+// Whether a cluster of CS CTAs can run the panel kernel (its attributes are
+// set on the first call; 16 CTAs only where the occupancy query finds room)
+template <class T, int CS>
+static bool panel_cluster_ok() {
+  static const bool ok = [] {
+    const int smem = pc_max_rpc<T, CS>(32) * 32 * (int)sizeof(cx<T>);
+    bool k = cudaFuncSetAttribute(k_getrf_panel_cluster<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
+             cudaSuccess;
+    if (k && CS > 8) {
+      k = cudaFuncSetAttribute(k_getrf_panel_cluster<T, CS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+          cudaSuccess;
+      if (k) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(CS, 1, 1);
+        cfg.blockDim = dim3(PC_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        int nclusters = 0;
+        k = cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_getrf_panel_cluster<T, CS>, &cfg) == cudaSuccess &&
+            nclusters >= 1;
+      }
+    }
+    (void)cudaGetLastError();  // a refused attribute or query leaves this size off, nothing else
+    return k;
+  }();
+  return ok;
+}
+
+template <class T, int CS>
+static int panel_cluster(const LUBatch<T>& f, int j0, int w, cudaStream_t st) {
+  const int rpc = (f.n - j0 + CS - 1) / CS;
+  k_getrf_panel_cluster<T, CS><<<f.batch * CS, PC_THREADS, (size_t)rpc * w * sizeof(cx<T>), st>>>(
+      f.A, f.n, f.stride, j0, w, rpc, f.ipiv, f.info);
+  QBG_LAUNCH_CHECK("k_getrf_panel_cluster");
+  return QBG_OK;
+}
+
+// CTAs per panel of w columns (0: the one-CTA kernel). automatic:
+//  * complex64: a cluster for batches of at most 4, where one CTA per panel
+//    leaves most SMs idle; for larger batches the one-CTA panels of several
+//    matrices already run beside other matrices' updates, and the cluster form
+//    measured slower (48 operators of 2048 in four stream parts: factor phase
+//    38.5 ms with clusters against 34.0 ms without).
+//  * complex128: one SM's FP64 pipe (2 FMAs per clock) bounds the panel, so the
+//    size is the one that spreads the batch's panels over the SMs best: waves
+//    of CTAs, one per SM, times the share of a panel a CTA does plus a tenth
+//    for the cluster's per-column exchange; the one-CTA kernel unless that is
+//    a fifth less. Measured, with the panels narrowed from 64 (32 in Beyn
+//    handles) to 32 columns: 24 operators of 1502 (4 CTAs each) 91.5 -> 67.6 ms
+//    for the whole Beyn call, a sweep of 16 operators of 1130 (8 CTAs) 63 -> 44
+//    ms, one of 200 operators of 512 (one CTA) 58 -> 57 ms.
+// set_lu_plan (or QBG_LU_CLUSTER=0 / =1 in the environment) forces either form.
+template <class T>
+static int panel_cluster_size(int n, int batch, int w) {
+  const int set = g_lu_cluster.load();
+  if (w > 64 || set == 0) return 0;
+  const int fits[4] = {n <= 2 * pc_max_rpc<T, 2>(w), n <= 4 * pc_max_rpc<T, 4>(w), n <= 8 * pc_max_rpc<T, 8>(w),
+                       n <= 16 * pc_max_rpc<T, 16>(w)};
+  if (sizeof(T) == 4) {
+    if (set < 0 && batch > 4) return 0;
+    if (fits[2] && panel_cluster_ok<T, 8>()) return 8;
+    return fits[3] && panel_cluster_ok<T, 16>() ? 16 : 0;
+  }
+  const bool ok[4] = {panel_cluster_ok<T, 2>(), panel_cluster_ok<T, 4>(), panel_cluster_ok<T, 8>(),
+                      panel_cluster_ok<T, 16>()};
+  double best = set == 1 ? 1e300 : 0.8 * ((batch + 151) / 152);
+  int cs = 0;
+  for (int i = 0; i < 4; ++i) {
+    const int c = 2 << i;
+    const double cost = (double)(((long long)batch * c + 151) / 152) * (1.0 / c + 0.1);
+    if (fits[i] && ok[i] && cost < best) {
+      best = cost;
+      cs = c;
+    }
+  }
+  return cs;
+}
+
 template <class T>
 static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first_panel = nullptr) {
   const int n = f.n, nb = f.nb, batch = f.batch;
@@ -1084,45 +1162,11 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
                                   (int)kPanelSmem));
     panel_attr[sizeof(T) == 8] = true;
   }
-  // panels of up to 64 columns and n <= 8 (or 16) * pc_max_rpc rows of a small
-  // batch (at most 4 matrices, where one CTA per panel leaves most SMs idle;
-  // for complex128 one SM's FP64 pipe takes ~1 ms per 500 x 64 panel) go to
-  // a cluster of CTAs. For larger batches the one-CTA panels of
-  // several matrices already run side by side with other matrices' updates,
-  // and the cluster form measured slower (48 operators of 2048 in four
-  // stream parts: factor phase 38.5 ms with clusters against 34.0 ms without).
-  // set_lu_plan (or QBG_LU_CLUSTER=0 / =1 in the environment) forces either form.
-  const int cluster_set = g_lu_cluster.load();
-  const bool cluster_on = cluster_set < 0 ? batch <= 4 : cluster_set == 1;
-  static bool cluster_attr[2] = {false, false};
-  static bool cluster16_ok[2] = {false, false};
-  if (cluster_on && nb <= 64 && !cluster_attr[sizeof(T) == 8]) {
-    QBG_CUDA(cudaFuncSetAttribute(k_getrf_panel_cluster<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  pc_max_rpc<T, 8>() * 64 * (int)sizeof(cx<T>)));
-    // 16-CTA clusters exist on this part as a non-portable size: allowed only
-    // when the occupancy query finds room for at least one
-    bool ok = cudaFuncSetAttribute(k_getrf_panel_cluster<T, 16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                  cudaSuccess &&
-              cudaFuncSetAttribute(k_getrf_panel_cluster<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   pc_max_rpc<T, 16>() * 64 * (int)sizeof(cx<T>)) == cudaSuccess;
-    if (ok) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(16, 1, 1);
-      cfg.blockDim = dim3(PC_THREADS, 1, 1);
-      cfg.dynamicSmemBytes = (size_t)pc_max_rpc<T, 16>() * 64 * sizeof(cx<T>);
-      int nclusters = 0;
-      ok = cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_getrf_panel_cluster<T, 16>, &cfg) == cudaSuccess &&
-           nclusters >= 1;
-    }
-    (void)cudaGetLastError();  // a refused attribute or query leaves 16-CTA clusters off, nothing else
-    cluster16_ok[sizeof(T) == 8] = ok;
-    cluster_attr[sizeof(T) == 8] = true;
-  }
-  const int pcs = !(cluster_on && nb <= 64)                  ? 0
-                  : n <= 8 * pc_max_rpc<T, 8>()               ? 8
-                  : (cluster16_ok[sizeof(T) == 8] && n <= 16 * pc_max_rpc<T, 16>()) ? 16
-                                                              : 0;
-  const bool use_cluster = pcs > 0;
+  // complex128 panels are 32 columns wide whatever the block size of the
+  // inverses: half of a 64-column panel's FP64 work is its second half's
+  // update, which the tensor cores do in a fraction of the time
+  const int pw = sizeof(T) == 8 ? std::min(nb, 32) : nb;
+  const int pcs = panel_cluster_size<T>(n, batch, pw);
   QBG_CUDA(cudaMemsetAsync(f.info, 0, sizeof(int) * batch, st));
   // two-level right-looking LU: panels of nb columns inside outer blocks of
   // LU_OUTER panels. A panel's updates reach only the columns of its outer
@@ -1133,40 +1177,52 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   // so the factors are those of the one-level algorithm.
   // panels per outer block: set_lu_plan (or QBG_LU_OUTER in the environment), 1..16, default 4
   const int LU_OUTER = g_lu_outer.load();
-  auto linv = [&](int j) { return f.Linv + (long long)(j / nb) * nb * nb; };
-  const long long sLinv = (long long)f.nblk * nb * nb;
-  for (int J0 = 0; J0 < n; J0 += LU_OUTER * nb) {
-    const int E = min(n, J0 + LU_OUTER * nb);  // outer block columns [J0, E)
-    for (int j0 = J0; j0 < E; j0 += nb) {
-      const int w = min(nb, n - j0);
-      if (use_cluster) {
-        const int rpc = (n - j0 + pcs - 1) / pcs;
-        const size_t smem = (size_t)rpc * 64 * sizeof(cx<T>);
-        if (pcs == 8)
-          k_getrf_panel_cluster<T, 8><<<batch * 8, PC_THREADS, smem, st>>>(f.A, n, f.stride, j0, nb, rpc, f.ipiv,
-                                                                           f.info);
-        else
-          k_getrf_panel_cluster<T, 16><<<batch * 16, PC_THREADS, smem, st>>>(f.A, n, f.stride, j0, nb, rpc, f.ipiv,
-                                                                             f.info);
-        QBG_LAUNCH_CHECK("k_getrf_panel_cluster");
+  // inverses of the pw x pw diagonal blocks of L, for the U rows
+  const int npw = (n + pw - 1) / pw;
+  cx<T>* Lp = f.Linv;
+  struct Scratch {
+    cx<T>* p = nullptr;
+    cudaStream_t st = nullptr;
+    ~Scratch() { if (p) dfree(p, st); }
+  } scratch;
+  if (pw != nb) {
+    QBG_TRY(dmalloc(&scratch.p, sizeof(cx<T>) * (size_t)npw * pw * pw * batch));
+    scratch.st = st;
+    Lp = scratch.p;
+  }
+  const size_t smp = (size_t)pw * pw * sizeof(cx<T>) * 5 / 4;
+  auto linv = [&](int j) { return Lp + (long long)(j / pw) * pw * pw; };
+  const long long sLinv = (long long)npw * pw * pw;
+  for (int J0 = 0; J0 < n; J0 += LU_OUTER * pw) {
+    const int E = min(n, J0 + LU_OUTER * pw);  // outer block columns [J0, E)
+    for (int j0 = J0; j0 < E; j0 += pw) {
+      const int w = min(pw, n - j0);
+      if (pcs == 2) {
+        QBG_TRY((panel_cluster<T, 2>(f, j0, w, st)));
+      } else if (pcs == 4) {
+        QBG_TRY((panel_cluster<T, 4>(f, j0, w, st)));
+      } else if (pcs == 8) {
+        QBG_TRY((panel_cluster<T, 8>(f, j0, w, st)));
+      } else if (pcs == 16) {
+        QBG_TRY((panel_cluster<T, 16>(f, j0, w, st)));
       } else if (smem_panel) {
         const size_t smem = (size_t)(n - j0) * sub * sizeof(cx<T>);
-        k_getrf_panel_smem<T><<<batch, 1024, smem, st>>>(f.A, n, f.stride, j0, nb, sub, f.ipiv, f.info);
+        k_getrf_panel_smem<T><<<batch, 1024, smem, st>>>(f.A, n, f.stride, j0, pw, sub, f.ipiv, f.info);
         QBG_LAUNCH_CHECK("k_getrf_panel_smem");
       } else {
-        k_getf2_panel<T><<<batch, 512, 0, st>>>(f.A, n, f.stride, j0, nb, f.ipiv, f.info);
+        k_getf2_panel<T><<<batch, 512, 0, st>>>(f.A, n, f.stride, j0, pw, f.ipiv, f.info);
         QBG_LAUNCH_CHECK("k_getf2_panel");
       }
       dim3 g2((n + 255) / 256, batch);
-      k_laswp<T><<<g2, 256, 0, st>>>(f.A, n, f.stride, j0, nb, f.ipiv);
+      k_laswp<T><<<g2, 256, 0, st>>>(f.A, n, f.stride, j0, pw, f.ipiv);
       QBG_LAUNCH_CHECK("k_laswp");
-      k_trtri<T, false><<<dim3(1, batch), 256, sm, st>>>(f.A, n, f.stride, nb, j0 / nb, f.Linv, f.nblk);
+      k_trtri<T, false><<<dim3(1, batch), 256, smp, st>>>(f.A, n, f.stride, pw, j0 / pw, Lp, npw);
       QBG_LAUNCH_CHECK("k_trtri lower");
       if (j0 == 0 && after_first_panel) QBG_CUDA(cudaEventRecord(after_first_panel, st));
       const int rin = E - j0 - w;  // columns of this outer block right of the panel
       if (rin > 0) {
         // U12 = inv(L11) A12 and A22 -= L21 U12 on the outer block's columns
-        int s = block_mul<T>(w, rin, linv(j0), nb, sLinv, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, st);
+        int s = block_mul<T>(w, rin, linv(j0), pw, sLinv, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, st);
         if (s) return s;
         s = gemm_sub<T>(n - j0 - w, rin, w, f.A + (j0 + w) + (long long)j0 * n, n, f.stride,
                         f.A + j0 + (long long)(j0 + w) * n, n, f.stride, f.A + (j0 + w) + (long long)(j0 + w) * n, n,
@@ -1177,9 +1233,9 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
     const int rest = n - E;
     if (rest > 0) {
       // U rows of the outer block on the trailing columns: U_b = inv(L_bb) (A_b - sum_{b'<b} L_bb' U_b')
-      for (int j0 = J0; j0 < E; j0 += nb) {
-        const int w = min(nb, E - j0);
-        int s = block_mul<T>(w, rest, linv(j0), nb, sLinv, f.A + j0 + (long long)E * n, n, f.stride, batch, st);
+      for (int j0 = J0; j0 < E; j0 += pw) {
+        const int w = min(pw, E - j0);
+        int s = block_mul<T>(w, rest, linv(j0), pw, sLinv, f.A + j0 + (long long)E * n, n, f.stride, batch, st);
         if (s) return s;
         const int below = E - j0 - w;
         if (below > 0) {
@@ -1194,6 +1250,10 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
                           n, f.stride, f.A + E + (long long)E * n, n, f.stride, batch, st);
       if (s) return s;
     }
+  }
+  if (pw != nb) {
+    k_trtri<T, false><<<dim3(f.nblk, batch), 256, sm, st>>>(f.A, n, f.stride, nb, 0, f.Linv, f.nblk);
+    QBG_LAUNCH_CHECK("k_trtri lower");
   }
   k_trtri<T, true><<<dim3(f.nblk, batch), 256, sm, st>>>(f.A, n, f.stride, nb, 0, f.Uinv, f.nblk);
   QBG_LAUNCH_CHECK("k_trtri upper");
