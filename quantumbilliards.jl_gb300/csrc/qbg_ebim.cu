@@ -350,6 +350,7 @@ struct Ebim {
   cudaEvent_t ev = nullptr;
   cxd *LU = nullptr, *dA = nullptr, *ddA = nullptr;
   cxd *C = nullptr, *CH = nullptr;  // A^-1 A' and its conjugate transpose
+  TcTall tall[2];                   // digit planes of C and CH, made by the first block iteration on them
   Dense64 D;                        // the library's FP64 LU of the matrix in LU
   std::vector<void*> tmp;
   ~Ebim() {
@@ -499,7 +500,24 @@ int block_eigs(Ebim& E, bool adjoint, int p, int nev, std::vector<zc>& mu, cxd* 
   QBG_TRY(E.alloc(&Y, sizeof(cxd) * np));
   QBG_TRY(E.alloc(&H, sizeof(cxd) * pp));
   QBG_TRY(E.alloc(&Xs, sizeof(cxd) * (size_t)p * nev));
-  QBG_TRY(E.alloc(&P, sizeof(cxd) * std::max<size_t>(tall_scratch(n, p), 1)));
+  // products on the tensor cores where the FP64 ones take longer than the four
+  // launches and the slice sum of a digit product: n^2 p complex FMAs at 2 FP64
+  // FMAs per clock and SM reach 50 us at n^2 p = 8e6 (n = 2048, p = 22: 1.40 ms
+  // in FP64, 0.08 ms here; the digits of the operator take 0.2 ms once)
+  const bool tc = (double)n * n * p >= 8e6;
+  TcTall& tall = E.tall[adjoint ? 1 : 0];
+  void* xmem = nullptr;
+  if (tc) {
+    if (!tall.TD) {
+      void* mem = nullptr;
+      QBG_TRY(E.alloc(&mem, tc_tall_bytes(n)));
+      QBG_TRY(tc_tall_prepare(tall, adjoint ? E.CH : E.C, n, mem, E.st));
+    }
+    QBG_TRY(E.alloc(&xmem, tc_tall_X_bytes(tall, p)));
+    QBG_TRY(E.alloc(&P, sizeof(cxd) * np * tc_tall_slices(tall)));
+  } else {
+    QBG_TRY(E.alloc(&P, sizeof(cxd) * std::max<size_t>(tall_scratch(n, p), 1)));
+  }
   QBG_TRY(E.alloc(&o.G, sizeof(cxd) * pp));
   QBG_TRY(E.alloc(&o.M, sizeof(cxd) * pp));
   QBG_TRY(E.alloc(&o.Wt, sizeof(cxd) * np));
@@ -522,7 +540,13 @@ int block_eigs(Ebim& E, bool adjoint, int p, int nev, std::vector<zc>& mu, cxd* 
   std::vector<int> order(p);
   for (int it = 0; it < MAXIT; ++it) {
     // Y = C Q, or C^H Q
-    QBG_TRY(gemm_nq(adjoint ? E.CH : E.C, Q, Y, n, p, P, E.st));
+    if (tc) {
+      QBG_TRY(tc_tall_product(tall, Q, p, xmem, P, E.st));
+      k_sum_slices<<<(unsigned)std::min<size_t>((np + 255) / 256, 4096), 256, 0, E.st>>>(P, tc_tall_slices(tall), np, Y);
+      QBG_LAUNCH_CHECK("k_sum_slices");
+    } else {
+      QBG_TRY(gemm_nq(adjoint ? E.CH : E.C, Q, Y, n, p, P, E.st));
+    }
     // Rayleigh-Ritz on the projection Q^H Y
     k_inner<<<p * p, 256, 0, E.st>>>(Q, Y, n, p, H);
     QBG_LAUNCH_CHECK("k_inner");
@@ -652,6 +676,7 @@ int ebim_run(Ebim& E, double k, double dk, int nev_req, int flags, int cap, doub
     }
     ++m;
   }
+  QBG_TRY(tc_check(E.st));
   *count = m;
   if (iters_out) {
     iters_out[0] = itr;

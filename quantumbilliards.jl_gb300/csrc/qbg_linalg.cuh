@@ -148,6 +148,20 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
 // FP64, the rest as above
 int tc_block_mul_f64(int w, int N, const cxd* A, long long lda, long long sA, cxd* X, long long ldx, long long sX,
                      int batch, cudaStream_t st);
+// A X for one n x n A and a few columns X, repeatedly (qbg_tc_resid.cu):
+// prepare takes A's digits into mem (tc_tall_bytes); a product (q columns, xmem
+// of tc_tall_X_bytes) writes tc_tall_slices partial products, n x q each, to P,
+// to be summed in order.
+struct TcTall {
+  int n = 0, MT = 0, KS = 0;
+  void* TD = nullptr;
+  int* erow = nullptr;
+};
+size_t tc_tall_bytes(int n);
+int tc_tall_prepare(TcTall& t, const cxd* A, int n, void* mem, cudaStream_t st);
+size_t tc_tall_X_bytes(const TcTall& t, int q);
+int tc_tall_slices(const TcTall& t);
+int tc_tall_product(const TcTall& t, const cxd* X, int q, void* xmem, cxd* P, cudaStream_t st);
 // device address of the tensor-core error flag (shared by the GEMM and the residual)
 int tc_error_ptr(int** p);
 

@@ -40,6 +40,7 @@
 // wait is bounded (1e9 SM cycles): on a timeout the CTA records an error,
 // waits (bounded) for the copies and MMAs it started, frees its TMEM and
 // returns without writing R.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
 #include "qbg_common.cuh"
@@ -618,7 +619,9 @@ __global__ void __launch_bounds__(256) k_x_prep_f64(const cxd* __restrict__ X, l
 // scales (for refinement sweeps whose correction is not the last)
 // P: digit planes per operand image (ND <= P); n: rows of T, V and R; ldv:
 // leading dimension of V and R (column l of row i at i + l ldv); Dg (optional,
-// the diagonal entries Dg[i ldd] of row i): R = diag(Dg) V + T X
+// the diagonal entries Dg[i ldd] of row i): R = diag(Dg) V + T X. nsplit > 1 (V
+// null): slice q of the k extent, kper stages, gives its own product T_q X_q at
+// R + (batch nsplit + q) sR
 template <int ND, int P>
 __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* __restrict__ TD,
                                                      const int* __restrict__ erow,
@@ -627,7 +630,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
                                                      const cxd* V, long long sV, cxd* R, long long sR, long long ldv,
                                                      unsigned long long* rmax, int* err,
                                                      const cxd* __restrict__ Dg = nullptr, long long sD = 0,
-                                                     long long ldd = 0) {
+                                                     long long ldd = 0, int kper = 0, int nsplit = 1) {
   constexpr int RA_TILE = RLay<P>::A_TILE, RB_TILE = RLay<P>::B_TILE, RSTAGE = RLay<P>::STAGE;
   // stages between exact flushes: a level of ND digits collects up to ND
   // pairs, so 16 stages (256 real k) keep eight-digit level sums below 2^23
@@ -641,8 +644,11 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int nt = blockIdx.x, mt = blockIdx.y;
-  const long long z = blockIdx.z;
+  const long long z = blockIdx.z / nsplit, zr = blockIdx.z;
   const int n0 = nt * RBN, m0 = mt * RBM;
+  const int kb = nsplit > 1 ? (int)(blockIdx.z % nsplit) * kper : 0;  // first stage of this slice
+  const int KSI = KS;                                                 // stages of an image
+  if (nsplit > 1) KS = min(KS - kb, kper);
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(r_smem_u32(tmem_slot)),
@@ -673,8 +679,8 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
   for (int c = 0; c < 2 * RCW; ++c) { acc_hi[c] = 0; acc_lo[c] = 0; }
 
   // thread 0: producer and MMA issuer
-  const unsigned char* ta = TD + (z * MT + mt) * (long long)KS * RA_TILE;
-  const unsigned char* xb = XD + (z * NT + nt) * (long long)KS * RB_TILE;
+  const unsigned char* ta = TD + ((z * MT + mt) * (long long)KSI + kb) * RA_TILE;
+  const unsigned char* xb = XD + ((z * NT + nt) * (long long)KSI + kb) * RB_TILE;
   int issued = 0, consumed = 0, committed = 0, freed = 0;
   bool good = (*abort_flag == 0);
   // the leading ND planes of each tile image (planes are stored most significant first)
@@ -788,7 +794,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
     if (i < n) {
       const int ei = erow[z * n + i];
       const cxd* Vb = V + z * sV;
-      cxd* Rb = R + z * sR;
+      cxd* Rb = R + zr * sR;
       const cxd dg = Dg ? Dg[z * sD + (long long)i * ldd] : cxd(0.0, 0.0);
 #pragma unroll
       for (int c = 0; c < RCW; ++c) {
@@ -796,7 +802,7 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
         if (col >= L) continue;  // full unroll keeps the sums in registers
         const int f = fcol[z * L + col];
         const long long e = (long long)i + (long long)col * ldv;
-        const cxd v = Vb[e];
+        const cxd v = V ? Vb[e] : cxd(0.0, 0.0);
         cxd r;
         if (ei == R_NONFINITE || f == R_NONFINITE) {
           r = cxd(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
@@ -804,9 +810,9 @@ __global__ void __launch_bounds__(RTHREADS, 1) k_resid_tc(const unsigned char* _
           const int e2 = ei + f - 7 * (ND + 1);
           const double re = fixed_to_f64<7 * (ND - 4)>(acc_hi[c], acc_lo[c], e2);
           const double im = fixed_to_f64<7 * (ND - 4)>(acc_hi[RCW + c], acc_lo[RCW + c], e2);
-          if (Dg) {
+          if (Dg || !V) {
             r = cxd(re, im);
-            cfma(r, dg, v);
+            if (Dg) cfma(r, dg, v);
           } else {
             r = cxd(v.re - re, v.im - im);
           }
@@ -1025,6 +1031,70 @@ int tc_gemm_sub_f64(int M, int N, int K, const cxd* A, long long lda, long long 
 int tc_block_mul_f64(int w, int N, const cxd* A, long long lda, long long sA, cxd* X, long long ldx, long long sX,
                      int batch, cudaStream_t st) {
   return tc_gemm_f64(w, N, w, A, lda, sA, X, ldx, sX, X, ldx, sX, batch, st, true);
+}
+
+// ---------------------------------------------------------------------------
+// A Y for one n x n A and a few columns, many times with the same A (the block
+// iterations of the EBIM step): the digit planes of A are made once; a product
+// then costs the MMAs of n / 128 row tiles over the k extent, cut into slices
+// so that about one CTA per SM takes part, and a fixed-order sum of the slices.
+// ---------------------------------------------------------------------------
+static int tall_kper(const TcTall& t) {
+  // slices of whole 16-stage flushes (256 real k), at most about 152 CTAs
+  const int slices = std::max(1, 152 / t.MT);
+  return ((t.KS + slices - 1) / slices + 15) / 16 * 16;
+}
+
+static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+size_t tc_tall_bytes(int n) {
+  const size_t MT = (n + RBM - 1) / RBM, KS = (2 * (size_t)n + RKS - 1) / RKS;
+  return up256(MT * KS * RLay<8>::A_TILE) + sizeof(int) * n;
+}
+
+int tc_tall_prepare(TcTall& t, const cxd* A, int n, void* mem, cudaStream_t st) {
+  constexpr int P = 8;
+  t.n = n;
+  t.MT = (n + RBM - 1) / RBM;
+  t.KS = (2 * n + RKS - 1) / RKS;
+  t.TD = mem;
+  t.erow = reinterpret_cast<int*>(static_cast<unsigned char*>(mem) + up256((size_t)t.MT * t.KS * RLay<P>::A_TILE));
+  QBG_CUDA(cudaFuncSetAttribute(k_resid_tc<P, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r_smem_bytes<P>()));
+  QBG_CUDA(cudaMemsetAsync(mem, 0, tc_tall_bytes(n), st));  // rows and k past the ends stay zero
+  k_a_rowexp_f64<<<dim3((n + 31) / 32, 1), dim3(32, 8), 0, st>>>(A, 0, n, n, n, t.erow);
+  QBG_LAUNCH_CHECK("k_a_rowexp_f64");
+  k_a_digits_f64<P><<<dim3((n + 31) / 32, (n + 31) / 32, 1), dim3(32, 8), 0, st>>>(
+      A, 0, n, n, n, t.MT, t.KS, t.erow, static_cast<unsigned char*>(t.TD));
+  QBG_LAUNCH_CHECK("k_a_digits_f64");
+  return QBG_OK;
+}
+
+size_t tc_tall_X_bytes(const TcTall& t, int q) {
+  return up256((size_t)(lp_of(q) / RBN) * t.KS * RLay<8>::B_TILE) + sizeof(int) * q;
+}
+
+int tc_tall_slices(const TcTall& t) {
+  const int kper = tall_kper(t);
+  return (t.KS + kper - 1) / kper;
+}
+
+int tc_tall_product(const TcTall& t, const cxd* X, int q, void* xmem, cxd* P_, cudaStream_t st) {
+  constexpr int P = 8;
+  const int n = t.n, Lp = lp_of(q), NT = Lp / RBN, kper = tall_kper(t), ns = tc_tall_slices(t);
+  int* derr = nullptr;
+  QBG_TRY(tc_error_ptr(&derr));
+  unsigned char* XD = static_cast<unsigned char*>(xmem);
+  const size_t dig = (size_t)NT * t.KS * RLay<P>::B_TILE;
+  int* fcol = reinterpret_cast<int*>(XD + up256(dig));
+  if (n % 8) QBG_CUDA(cudaMemsetAsync(XD, 0, dig, st));  // k past n
+  k_x_colexp<<<dim3(q, 1), 256, 0, st>>>(X, 0, n, n, q, fcol);
+  QBG_LAUNCH_CHECK("k_x_colexp");
+  k_x_digits<P><<<dim3((n + 255) / 256, Lp, 1), 256, 0, st>>>(X, 0, n, n, q, NT, t.KS, fcol, XD);
+  QBG_LAUNCH_CHECK("k_x_digits");
+  k_resid_tc<P, P><<<dim3(NT, t.MT, ns), RTHREADS, r_smem_bytes<P>(), st>>>(
+      static_cast<const unsigned char*>(t.TD), t.erow, XD, fcol, n, q, t.MT, NT, t.KS, nullptr, 0, P_, (long long)n * q, n, nullptr, derr, nullptr, 0, 0, kper, ns);
+  QBG_LAUNCH_CHECK("k_resid_tc");
+  return QBG_OK;
 }
 
 }  // namespace qbg
