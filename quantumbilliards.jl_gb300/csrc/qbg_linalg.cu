@@ -692,6 +692,277 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(PC_THREADS)
   store_block<T>(a + (j0 + r0) + (long long)j0 * n, n, P, rpc, rows, w, tid, PC_THREADS);
 }
 
+// ---------------------------------------------------------------------------
+// complex64 panel on a cluster of CS CTAs per matrix, 8-column sub-panels in
+// registers. The m x w panel (w <= 64) is in the CTAs' shared memory, rows in
+// blocks of rpc = ceil(m / CS); a thread owns rows tid and tid + 256 of its CTA
+// and keeps their eight sub-panel columns in registers while it is factored.
+//
+// Column step: warp maxima by redux (key = bits of |re| + |im|, plus one; 0 for
+// none, so a NaN is never a candidate), one block barrier, the warp that owns
+// the block's candidate pushes its eight values to every CTA, the owner of the
+// diagonal row pushes that row, one cluster barrier; then every thread picks
+// the pivot from the CS candidates, the two owners exchange the rows in
+// registers and every row is updated in registers. Push buffers alternate by
+// column parity as in k_getrf_panel_cluster.
+// Sub-panel step: the eight interchanges, composed to at most 16 moved rows,
+// reach the panel's other columns by pushes into the destination CTA, the eight
+// new top rows by pushes into every CTA (one cluster barrier); each CTA solves
+// U12 = inv(L11) A12 and every thread updates its rows by the rank-8 product,
+// multipliers in registers.
+// The factors, pivots (first index on ties) and info are those of
+// column-by-column partial pivoting.
+//
+// Bound by latency: one block and one cluster barrier per column, about 1.6 us.
+// Measured per 64-column panel: 145-160 us at up to 3200 rows, 190 us at 5000
+// (16 CTAs); the one-CTA kernel takes 340-460 us at 2048 rows, the cluster form
+// that keeps the panel in shared memory column by column 190-340 us.
+// ---------------------------------------------------------------------------
+constexpr int FP_T = 256, FP_SB = 8;
+constexpr int FP_ROWS = 400;  // rows per CTA: 64 columns in 200 KB (at most 2 FP_T)
+
+template <int CS>
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(FP_T)
+    k_getrf_panel_f32(cxf* A, int n, long long stride, int j0, int nb, int rpc, int* ipiv, int* info) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char smraw[];
+  cxf* P = reinterpret_cast<cxf*>(smraw);  // column c of the own rows at P + c * rpc
+  __shared__ __align__(16) cxf crow[2][CS][FP_SB];  // candidate rows pushed by every CTA
+  __shared__ __align__(16) cxf drow[2][FP_SB];      // the diagonal row
+  __shared__ uint2 cand[2][CS];                     // key and row of the candidates
+  __shared__ __align__(16) cxf mine[2][FP_SB];      // this CTA's candidate row, its diagonal row
+  __shared__ unsigned wkey[2][FP_T / 32];
+  __shared__ int wrow[2][FP_T / 32];
+  __shared__ cxf stg[2 * FP_SB][64];  // moved rows that come to this CTA
+  __shared__ cxf top[FP_SB][64];      // the sub-panel's top rows, columns right of it
+  __shared__ __align__(16) cxf Us[64][FP_SB];
+  __shared__ cxf L11[FP_SB][FP_SB];
+  __shared__ int tpos[2 * FP_SB], tsrc[2 * FP_SB], tcnt;
+  const int rank = (int)cl.block_rank();
+  const int mat = blockIdx.x / CS;
+  cxf* a = A + (long long)mat * stride;
+  int* piv = ipiv + (long long)mat * n;
+  const int m = n - j0, w = min(nb, m);
+  const int r0 = rank * rpc, rows = max(0, min(rpc, m - r0));
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  load_block<float>(P, rpc, a + (j0 + r0) + (long long)j0 * n, n, rows, w, tid, FP_T);
+  cl.sync();  // the panel is loaded; every CTA of the cluster runs before the first remote store
+  for (int s0 = 0; s0 < w; s0 += FP_SB) {
+    const int sw = min(FP_SB, w - s0);
+    cxf v[2][FP_SB];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int q = 0; q < FP_SB; ++q) {
+        const int i = tid + FP_T * j;
+        v[j][q] = (i < rows && q < sw) ? P[(s0 + q) * rpc + i] : cxf(0.f, 0.f);
+      }
+    int pos = -1, src = -1, cnt = 0;  // moved rows: lane t of every warp holds entry t
+#pragma unroll
+    for (int c = 0; c < FP_SB; ++c) {
+      if (c >= sw) break;
+      const int gc = s0 + c, buf = c & 1;
+      // candidate of the block
+      unsigned key = 0;
+      int row = 0x7fffffff;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int i = tid + FP_T * j, gr = r0 + i;
+        if (i < rows && gr >= gc) {
+          const float x = fabsf(v[j][c].re) + fabsf(v[j][c].im);
+          const unsigned k = x == x ? __float_as_uint(x) + 1u : 0u;
+          if (k > key) {
+            key = k;
+            row = gr;
+          }
+        }
+      }
+      unsigned mk = __reduce_max_sync(0xffffffffu, key);
+      int mr = __reduce_min_sync(0xffffffffu, key == mk ? row : 0x7fffffff);
+      if (lane == 0) {
+        wkey[buf][wid] = mk;
+        wrow[buf][wid] = mr;
+      }
+      __syncthreads();
+      key = lane < FP_T / 32 ? wkey[buf][lane] : 0u;
+      row = lane < FP_T / 32 ? wrow[buf][lane] : 0x7fffffff;
+      mk = __reduce_max_sync(0xffffffffu, key);
+      mr = __reduce_min_sync(0xffffffffu, key == mk ? row : 0x7fffffff);
+      if (mk == 0u) {
+        if (wid == 0 && lane < CS) *cl.map_shared_rank(&cand[buf][rank], lane) = make_uint2(0u, 0x7fffffffu);
+      } else if (((mr - r0) & (FP_T - 1)) >> 5 == wid) {  // this warp owns the candidate
+        const int i = mr - r0;
+        if (lane == (i & 31)) {
+#pragma unroll
+          for (int q = 0; q < FP_SB; ++q) mine[0][q] = i < FP_T ? v[0][q] : v[1][q];
+        }
+        __syncwarp();
+        for (int e = lane; e < CS * 5; e += 32) {
+          const int peer = e / 5, part = e % 5;
+          if (part < 4)
+            reinterpret_cast<float4*>(cl.map_shared_rank(&crow[buf][rank][0], peer))[part] =
+                reinterpret_cast<const float4*>(&mine[0][0])[part];
+          else
+            *cl.map_shared_rank(&cand[buf][rank], peer) = make_uint2(mk, (unsigned)mr);
+        }
+      }
+      if (gc >= r0 && gc < r0 + rows && ((gc - r0) & (FP_T - 1)) >> 5 == wid) {  // owner of the diagonal row
+        const int i = gc - r0;
+        if (lane == (i & 31)) {
+#pragma unroll
+          for (int q = 0; q < FP_SB; ++q) mine[1][q] = i < FP_T ? v[0][q] : v[1][q];
+        }
+        __syncwarp();
+        for (int e = lane; e < CS * 4; e += 32)
+          reinterpret_cast<float4*>(cl.map_shared_rank(&drow[buf][0], e / 4))[e % 4] =
+              reinterpret_cast<const float4*>(&mine[1][0])[e % 4];
+      }
+      cl.sync();  // candidates and the diagonal row of column gc everywhere
+      key = lane < CS ? cand[buf][lane].x : 0u;
+      row = lane < CS ? (int)cand[buf][lane].y : 0x7fffffff;
+      mk = __reduce_max_sync(0xffffffffu, key);
+      int p = __reduce_min_sync(0xffffffffu, key == mk ? row : 0x7fffffff);
+      const cxf* pr = mk ? crow[buf][p / rpc] : drow[buf];
+      if (!mk) p = gc;  // a NaN column: no interchange
+      cxf prow[FP_SB];
+#pragma unroll
+      for (int q = 0; q < FP_SB; q += 2) {
+        const float4 t = *reinterpret_cast<const float4*>(pr + q);
+        prow[q] = cxf(t.x, t.y);
+        prow[q + 1] = cxf(t.z, t.w);
+      }
+      if (rank == 0 && tid == 0) {
+        piv[j0 + gc] = j0 + p;
+        if (mk <= 1u && info[mat] == 0) info[mat] = j0 + gc + 1;  // none, or an exact zero
+      }
+      if (tid == 0) {
+#pragma unroll
+        for (int q = 0; q < FP_SB; ++q)
+          if (q < c) L11[c][q] = prow[q];
+      }
+      if (p != gc) {
+        unsigned b = __ballot_sync(0xffffffffu, pos == gc);
+        const int i1 = b ? __ffs(b) - 1 : cnt++;
+        if (!b && lane == i1) pos = src = gc;
+        b = __ballot_sync(0xffffffffu, pos == p);
+        const int i2 = b ? __ffs(b) - 1 : cnt++;
+        if (!b && lane == i2) pos = src = p;
+        const int x1 = __shfl_sync(0xffffffffu, src, i1), x2 = __shfl_sync(0xffffffffu, src, i2);
+        if (lane == i1) src = x2;
+        if (lane == i2) src = x1;
+      }
+      const cxf pv = prow[c];
+      const bool nz = pv.re != 0.f || pv.im != 0.f;
+      const cxf inv = nz ? cinv(pv) : cxf(1.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int gr = r0 + tid + FP_T * j;
+        if (gr == gc) {
+#pragma unroll
+          for (int q = 0; q < FP_SB; ++q) v[j][q] = prow[q];
+        } else if (gr == p) {
+#pragma unroll
+          for (int q = 0; q < FP_SB; ++q) v[j][q] = drow[buf][q];
+        }
+        if (gr > gc) {
+          const cxf l = nz ? v[j][c] * inv : v[j][c];
+          v[j][c] = l;
+#pragma unroll
+          for (int q = 0; q < FP_SB; ++q)
+            if (q > c) cfms(v[j][q], l, prow[q]);
+        }
+      }
+    }
+    // the factored columns back to shared memory
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int q = 0; q < FP_SB; ++q) {
+        const int i = tid + FP_T * j;
+        if (i < rows && q < sw) P[(s0 + q) * rpc + i] = v[j][q];
+      }
+    if (wid == 0) {
+      if (lane < cnt) {
+        tpos[lane] = pos;
+        tsrc[lane] = src;
+      }
+      if (lane == 0) tcnt = cnt;
+    }
+    __syncthreads();
+    // moved rows to their new owners, the new top rows to everyone
+    const int s1 = s0 + sw, nr = w - s1;
+    {
+      const int col = tid & 63, g = tid >> 6;
+      const bool other = col < w && (col < s0 || col >= s1);
+      if (other)
+        for (int t = g; t < tcnt; t += FP_T / 64) {
+          const int x = tsrc[t];
+          if (x >= r0 && x < r0 + rows) *cl.map_shared_rank(&stg[t][col], tpos[t] / rpc) = P[col * rpc + (x - r0)];
+        }
+      if (col >= s1 && col < w)
+        for (int k = g; k < sw; k += FP_T / 64) {
+          int x = s0 + k;
+          for (int t = 0; t < tcnt; ++t)
+            if (tpos[t] == s0 + k) x = tsrc[t];
+          if (x >= r0 && x < r0 + rows) {
+            const cxf e = P[col * rpc + (x - r0)];
+            for (int peer = 0; peer < CS; ++peer) *cl.map_shared_rank(&top[k][col], peer) = e;
+          }
+        }
+    }
+    cl.sync();
+    {
+      const int col = tid & 63, g = tid >> 6;
+      if (col < w && (col < s0 || col >= s1))
+        for (int t = g; t < tcnt; t += FP_T / 64) {
+          const int x = tpos[t];
+          if (x >= r0 && x < r0 + rows) P[col * rpc + (x - r0)] = stg[t][col];
+        }
+      if (tid < nr) {  // U12, one thread per column
+        cxf x[FP_SB];
+#pragma unroll
+        for (int k = 0; k < FP_SB; ++k) {
+          if (k < sw) {
+            x[k] = top[k][s1 + tid];
+#pragma unroll
+            for (int l = 0; l < FP_SB; ++l)
+              if (l < k) cfms(x[k], L11[k][l], x[l]);
+          } else {
+            x[k] = cxf(0.f, 0.f);
+          }
+          Us[tid][k] = x[k];
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = tid + FP_T * j, gr = r0 + i;
+      if (i >= rows || gr < s0) continue;
+      cxf* pc = P + s1 * rpc + i;
+      if (gr < s1) {
+        for (int q = 0; q < nr; ++q) pc[q * rpc] = Us[q][gr - s0];
+      } else {
+#pragma unroll 2
+        for (int q = 0; q < nr; ++q) {
+          cxf x = pc[q * rpc];
+#pragma unroll
+          for (int k = 0; k < FP_SB; k += 2) {
+            const float4 u = *reinterpret_cast<const float4*>(&Us[q][k]);
+            cfms(x, v[j][k], cxf(u.x, u.y));
+            cfms(x, v[j][k + 1], cxf(u.z, u.w));
+          }
+          pc[q * rpc] = x;
+        }
+      }
+    }
+    // Us, L11 and the permutation are rewritten only after the next block barrier
+    __syncthreads();
+  }
+  store_block<float>(a + (j0 + r0) + (long long)j0 * n, n, P, rpc, rows, w, tid, FP_T);
+}
+
 // row interchanges of one panel on the columns outside the panel
 template <class T>
 __global__ void k_laswp(cx<T>* A, int n, long long stride, int j0, int nb, const int* ipiv) {
@@ -1064,48 +1335,48 @@ static int block_mul(int w, int N, const cx<T>* A, long long lda, long long sA, 
   return gemm_batched<T>(w, N, w, cx<T>(1, 0), A, lda, sA, X, ldx, sX, cx<T>(0, 0), X, ldx, sX, batch, st);
 }
 
-// Whether a cluster of CS CTAs can run the panel kernel (its attributes are
-// set on the first call; 16 CTAs only where the occupancy query finds room)
-template <class T, int CS>
-static bool panel_cluster_ok() {
-  static const bool ok = [] {
-    const int smem = pc_max_rpc<T, CS>(32) * 32 * (int)sizeof(cx<T>);
-    bool k = cudaFuncSetAttribute(k_getrf_panel_cluster<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) ==
-             cudaSuccess;
-    if (k && CS > 8) {
-      k = cudaFuncSetAttribute(k_getrf_panel_cluster<T, CS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-          cudaSuccess;
-      if (k) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(CS, 1, 1);
-        cfg.blockDim = dim3(PC_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = (size_t)smem;
-        int nclusters = 0;
-        k = cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_getrf_panel_cluster<T, CS>, &cfg) == cudaSuccess &&
-            nclusters >= 1;
-      }
+// Whether clusters of cs CTAs can run the kernel with smem bytes of dynamic
+// shared memory (its attributes are set here; more than 8 CTAs only where the
+// occupancy query finds room)
+static bool cluster_kernel_ok(const void* kernel, int cs, int threads, int smem) {
+  bool k = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  if (k && cs > 8) {
+    k = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (k) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(cs, 1, 1);
+      cfg.blockDim = dim3(threads, 1, 1);
+      cfg.dynamicSmemBytes = (size_t)smem;
+      int nclusters = 0;
+      k = cudaOccupancyMaxActiveClusters(&nclusters, kernel, &cfg) == cudaSuccess && nclusters >= 1;
     }
-    (void)cudaGetLastError();  // a refused attribute or query leaves this size off, nothing else
-    return k;
-  }();
+  }
+  (void)cudaGetLastError();  // a refused attribute or query leaves this size off, nothing else
+  return k;
+}
+
+template <int CS>
+static bool panel_cluster_ok() {
+  static const bool ok = cluster_kernel_ok((const void*)k_getrf_panel_cluster<double, CS>, CS, PC_THREADS,
+                                           pc_max_rpc<double, CS>(32) * 32 * (int)sizeof(cxd));
   return ok;
 }
 
-template <class T, int CS>
-static int panel_cluster(const LUBatch<T>& f, int j0, int w, cudaStream_t st) {
+template <int CS>
+static int panel_cluster(const LUBatch<double>& f, int j0, int w, cudaStream_t st) {
   const int rpc = (f.n - j0 + CS - 1) / CS;
-  k_getrf_panel_cluster<T, CS><<<f.batch * CS, PC_THREADS, (size_t)rpc * w * sizeof(cx<T>), st>>>(
+  k_getrf_panel_cluster<double, CS><<<f.batch * CS, PC_THREADS, (size_t)rpc * w * sizeof(cxd), st>>>(
       f.A, f.n, f.stride, j0, w, rpc, f.ipiv, f.info);
   QBG_LAUNCH_CHECK("k_getrf_panel_cluster");
   return QBG_OK;
 }
 
-// CTAs per panel of w columns (0: the one-CTA kernel). automatic:
-//  * complex64: a cluster for batches of at most 4, where one CTA per panel
-//    leaves most SMs idle; for larger batches the one-CTA panels of several
-//    matrices already run beside other matrices' updates, and the cluster form
-//    measured slower (48 operators of 2048 in four stream parts: factor phase
-//    38.5 ms with clusters against 34.0 ms without).
+// CTAs per panel of w columns and m rows (0: the one-CTA kernel). automatic:
+//  * complex64: the smallest cluster of k_getrf_panel_f32 that holds the rows
+//    left (its barriers cost more than its updates, so more CTAs gain nothing),
+//    also for large batches: a Beyn call on 48 operators of 2048 takes 60.7 ms
+//    with it and 63.2 ms with one-CTA panels, on 8 resident operators of 5002
+//    165 ms against 251 ms, on 384 of 1024 the same 211 ms.
 //  * complex128: one SM's FP64 pipe (2 FMAs per clock) bounds the panel, so the
 //    size is the one that spreads the batch's panels over the SMs best: waves
 //    of CTAs, one per SM, times the share of a panel a CTA does plus a tenth
@@ -1115,30 +1386,70 @@ static int panel_cluster(const LUBatch<T>& f, int j0, int w, cudaStream_t st) {
 //    for the whole Beyn call, a sweep of 16 operators of 1130 (8 CTAs) 63 -> 44
 //    ms, one of 200 operators of 512 (one CTA) 58 -> 57 ms.
 // set_lu_plan (or QBG_LU_CLUSTER=0 / =1 in the environment) forces either form.
-template <class T>
-static int panel_cluster_size(int n, int batch, int w) {
+static int panel_cluster_size_f64(int n, int batch, int w) {
   const int set = g_lu_cluster.load();
   if (w > 64 || set == 0) return 0;
-  const int fits[4] = {n <= 2 * pc_max_rpc<T, 2>(w), n <= 4 * pc_max_rpc<T, 4>(w), n <= 8 * pc_max_rpc<T, 8>(w),
-                       n <= 16 * pc_max_rpc<T, 16>(w)};
-  if (sizeof(T) == 4) {
-    if (set < 0 && batch > 4) return 0;
-    if (fits[2] && panel_cluster_ok<T, 8>()) return 8;
-    return fits[3] && panel_cluster_ok<T, 16>() ? 16 : 0;
-  }
-  const bool ok[4] = {panel_cluster_ok<T, 2>(), panel_cluster_ok<T, 4>(), panel_cluster_ok<T, 8>(),
-                      panel_cluster_ok<T, 16>()};
+  const bool ok[4] = {n <= 2 * pc_max_rpc<double, 2>(w) && panel_cluster_ok<2>(),
+                      n <= 4 * pc_max_rpc<double, 4>(w) && panel_cluster_ok<4>(),
+                      n <= 8 * pc_max_rpc<double, 8>(w) && panel_cluster_ok<8>(),
+                      n <= 16 * pc_max_rpc<double, 16>(w) && panel_cluster_ok<16>()};
   double best = set == 1 ? 1e300 : 0.8 * ((batch + 151) / 152);
   int cs = 0;
   for (int i = 0; i < 4; ++i) {
     const int c = 2 << i;
     const double cost = (double)(((long long)batch * c + 151) / 152) * (1.0 / c + 0.1);
-    if (fits[i] && ok[i] && cost < best) {
+    if (ok[i] && cost < best) {
       best = cost;
       cs = c;
     }
   }
   return cs;
+}
+
+template <int CS>
+static bool panel_f32_ok() {
+  static const bool ok = cluster_kernel_ok((const void*)k_getrf_panel_f32<CS>, CS, FP_T, FP_ROWS * 64 * (int)sizeof(cxf));
+  return ok;
+}
+
+// 0: the one-CTA kernel
+static int panel_cluster_size_f32(int m, int w) {
+  if (w > 64 || g_lu_cluster.load() == 0) return 0;
+  if (m <= FP_ROWS && panel_f32_ok<1>()) return 1;
+  if (m <= 2 * FP_ROWS && panel_f32_ok<2>()) return 2;
+  if (m <= 4 * FP_ROWS && panel_f32_ok<4>()) return 4;
+  if (m <= 8 * FP_ROWS && panel_f32_ok<8>()) return 8;
+  return m <= 16 * FP_ROWS && panel_f32_ok<16>() ? 16 : 0;
+}
+
+template <int CS>
+static int panel_f32(const LUBatch<float>& f, int j0, int w, cudaStream_t st) {
+  const int rpc = (f.n - j0 + CS - 1) / CS;
+  k_getrf_panel_f32<CS><<<f.batch * CS, FP_T, (size_t)rpc * w * sizeof(cxf), st>>>(f.A, f.n, f.stride, j0, w, rpc,
+                                                                                  f.ipiv, f.info);
+  QBG_LAUNCH_CHECK("k_getrf_panel_f32");
+  return QBG_OK;
+}
+
+// the panel of columns j0 .. j0 + w - 1 on a cluster; false: left to the one-CTA kernels
+static bool panel_on_cluster(const LUBatch<float>& f, int j0, int w, cudaStream_t st, int* status) {
+  switch (panel_cluster_size_f32(f.n - j0, w)) {
+    case 1: *status = panel_f32<1>(f, j0, w, st); return true;
+    case 2: *status = panel_f32<2>(f, j0, w, st); return true;
+    case 4: *status = panel_f32<4>(f, j0, w, st); return true;
+    case 8: *status = panel_f32<8>(f, j0, w, st); return true;
+    case 16: *status = panel_f32<16>(f, j0, w, st); return true;
+    default: return false;
+  }
+}
+static bool panel_on_cluster(const LUBatch<double>& f, int j0, int w, cudaStream_t st, int* status) {
+  switch (panel_cluster_size_f64(f.n, f.batch, w)) {
+    case 2: *status = panel_cluster<2>(f, j0, w, st); return true;
+    case 4: *status = panel_cluster<4>(f, j0, w, st); return true;
+    case 8: *status = panel_cluster<8>(f, j0, w, st); return true;
+    case 16: *status = panel_cluster<16>(f, j0, w, st); return true;
+    default: return false;
+  }
 }
 
 template <class T>
@@ -1166,7 +1477,6 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   // inverses: half of a 64-column panel's FP64 work is its second half's
   // update, which the tensor cores do in a fraction of the time
   const int pw = sizeof(T) == 8 ? std::min(nb, 32) : nb;
-  const int pcs = panel_cluster_size<T>(n, batch, pw);
   QBG_CUDA(cudaMemsetAsync(f.info, 0, sizeof(int) * batch, st));
   // two-level right-looking LU: panels of nb columns inside outer blocks of
   // LU_OUTER panels. A panel's updates reach only the columns of its outer
@@ -1197,14 +1507,9 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
     const int E = min(n, J0 + LU_OUTER * pw);  // outer block columns [J0, E)
     for (int j0 = J0; j0 < E; j0 += pw) {
       const int w = min(pw, n - j0);
-      if (pcs == 2) {
-        QBG_TRY((panel_cluster<T, 2>(f, j0, w, st)));
-      } else if (pcs == 4) {
-        QBG_TRY((panel_cluster<T, 4>(f, j0, w, st)));
-      } else if (pcs == 8) {
-        QBG_TRY((panel_cluster<T, 8>(f, j0, w, st)));
-      } else if (pcs == 16) {
-        QBG_TRY((panel_cluster<T, 16>(f, j0, w, st)));
+      int ps = QBG_OK;
+      if (panel_on_cluster(f, j0, w, st, &ps)) {
+        QBG_TRY(ps);
       } else if (smem_panel) {
         const size_t smem = (size_t)(n - j0) * sub * sizeof(cx<T>);
         k_getrf_panel_smem<T><<<batch, 1024, smem, st>>>(f.A, n, f.stride, j0, pw, sub, f.ipiv, f.info);
