@@ -2227,6 +2227,87 @@ int launch_kress_column(double* out, int N, cudaStream_t st) {
   return QBG_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Direct FP64 assembly of full operators by pairs: a CTA takes a pair of
+// 16 x 16 tiles (bi <= bj), a thread one pair of nodes (i, j), and forms both
+// entries (i, j) and (j, i), whose distance, log term and Bessel values are the
+// same; the mirrored tile goes through shared memory so that both are stored
+// with consecutive rows. Bound by FP64 issue, which the shared values halve.
+// Measured, entries one by one before: 24 real k of a 602-node DLP 1.53 -> 0.87
+// ms, A, A', A'' of a 1030-node CFIE 0.53 -> 0.39 ms.
+// ---------------------------------------------------------------------------
+constexpr int SYM_T = 16;
+
+template <int FORM, int DERIV>
+__global__ void __launch_bounds__(SYM_T* SYM_T) k_assemble_fp64_sym(GeomDev g, const cxd* __restrict__ ks, int nk,
+                                                                    int kchunk, cxd* const* __restrict__ outs,
+                                                                    long long ld) {
+  constexpr int NV = DERIV ? 3 : 1;
+  __shared__ cxd sm[NV][SYM_T][SYM_T + 1];
+  const int2 bp = tile_pair(blockIdx.x);
+  const int tx = threadIdx.x % SYM_T, ty = threadIdx.x / SYM_T;
+  const int i = bp.x * SYM_T + tx, j = bp.y * SYM_T + ty;
+  const bool inb = i < g.n && j < g.n, diag = inb && i == j, act = inb && (bp.x < bp.y || i < j);
+  // the mirrored tile's entry this thread stores: row j0 + tx, column i0 + ty
+  const int mr = bp.y * SYM_T + tx, mc = bp.x * SYM_T + ty;
+  const bool mst = mr < g.n && mc < g.n && (bp.x < bp.y || tx > ty);
+  const size_t off = (size_t)i + (size_t)j * (size_t)ld, moff = (size_t)mr + (size_t)mc * (size_t)ld;
+  PairGeom a, b;
+  bool zero = false;
+  if (act) {
+    pair_geom_sym(g, i, j, a, b);
+    zero = FORM == 1 && !a.same && a.r * a.r <= 4.93038065763132e-32;  // as in k_assemble_fp64
+  }
+  const int q1 = min(nk, ((int)blockIdx.z + 1) * kchunk);
+  for (int q = blockIdx.z * kchunk; q < q1; ++q) {
+    const cxd k = ks[q];
+    cxd F[NV], M[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) F[v] = M[v] = cxd(0.0, 0.0);
+    if (diag) {
+      F[0] = diag_fp64<FORM>(g, i, k);
+      if (DERIV) diag_derivs<FORM>(g, i, k, &F[NV > 1 ? 1 : 0], &F[NV > 2 ? 2 : 0]);
+    } else if (act && !zero) {
+      if (k.im == 0.0 && k.re > 0.0) {
+        const Bessel01r br = bessel01_real(a.r * k.re);
+        entry_vals_real<FORM, DERIV>(a, k.re, br, &F[0], &F[NV > 1 ? 1 : 0], &F[NV > 2 ? 2 : 0]);
+        entry_vals_real<FORM, DERIV>(b, k.re, br, &M[0], &M[NV > 1 ? 1 : 0], &M[NV > 2 ? 2 : 0]);
+      } else {
+        Bessel01d bc = bessel01(a.r * k);
+        if (k.im == 0.0) bc.j0.im = bc.j1.im = 0.0;
+        entry_vals<FORM, DERIV>(a, k, bc.h0(), bc.h1(), bc.j0, bc.j1, &F[0], &F[NV > 1 ? 1 : 0], &F[NV > 2 ? 2 : 0]);
+        entry_vals<FORM, DERIV>(b, k, bc.h0(), bc.h1(), bc.j0, bc.j1, &M[0], &M[NV > 1 ? 1 : 0], &M[NV > 2 ? 2 : 0]);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      if (act || diag) outs[v * nk + q][off] = F[v];
+      sm[v][ty][tx] = M[v];
+    }
+    __syncthreads();
+    if (mst)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) outs[v * nk + q][moff] = sm[v][tx][ty];
+    __syncthreads();
+  }
+}
+
+template <int FORM, int DERIV>
+static void launch_fp64(const GeomDev& g, const cxd* ks, int nk, cxd* const* outs, long long ld, cudaStream_t st) {
+  // by pairs from 100 tile pairs on (the k split over z where the tiles alone do
+  // not fill the device); smaller operators by entries, 64 to a CTA, since there
+  // the number of busy SMs counts: one k, the call with its copies, entries
+  // against pairs, n = 128 26 / 35 us, 192 32 / 35, 224 38 / 35, 400 73 / 61
+  const int nt = (g.n + SYM_T - 1) / SYM_T, tiles = nt * (nt + 1) / 2;
+  if ((long long)tiles * nk >= 100) {
+    const int nz = std::min(std::min(nk, std::max(1, 608 / tiles)), 65535), kchunk = (nk + nz - 1) / nz;
+    k_assemble_fp64_sym<FORM, DERIV><<<dim3(tiles, 1, (nk + kchunk - 1) / kchunk), SYM_T * SYM_T, 0, st>>>(
+        g, ks, nk, kchunk, outs, ld);
+  } else {
+    k_assemble_fp64<FORM, DERIV><<<dim3((g.n + 31) / 32, (g.n + 1) / 2), dim3(32, 2), 0, st>>>(g, ks, nk, outs, ld);
+  }
+}
+
 int launch_assemble(const GeomDev& g, const cxd* ks, int nk, int deriv, int prec, void* const* outs_dev,
                     long long ld, cudaStream_t st, void* const* lo_outs_dev) {
   const bool reduced = (g.m != g.n);
@@ -2253,16 +2334,13 @@ int launch_assemble(const GeomDev& g, const cxd* ks, int nk, int deriv, int prec
     return QBG_OK;
   }
   if (prec == QBG_PREC_FP64) {
+    cxd* const* outs = (cxd* const*)outs_dev;
     if (g.form == 0) {
-      if (deriv)
-        k_assemble_fp64<0, 1><<<grd, blk, 0, st>>>(g, ks, nk, (cxd* const*)outs_dev, ld);
-      else
-        k_assemble_fp64<0, 0><<<grd, blk, 0, st>>>(g, ks, nk, (cxd* const*)outs_dev, ld);
+      if (deriv) launch_fp64<0, 1>(g, ks, nk, outs, ld, st);
+      else launch_fp64<0, 0>(g, ks, nk, outs, ld, st);
     } else {
-      if (deriv)
-        k_assemble_fp64<1, 1><<<grd, blk, 0, st>>>(g, ks, nk, (cxd* const*)outs_dev, ld);
-      else
-        k_assemble_fp64<1, 0><<<grd, blk, 0, st>>>(g, ks, nk, (cxd* const*)outs_dev, ld);
+      if (deriv) launch_fp64<1, 1>(g, ks, nk, outs, ld, st);
+      else launch_fp64<1, 0>(g, ks, nk, outs, ld, st);
     }
     QBG_LAUNCH_CHECK("k_assemble_fp64");
     return QBG_OK;
