@@ -1422,8 +1422,11 @@ __global__ void k_cheb_df_tables(ChebTables t) {
 // 1/r near rmin (7695 against 863 J panels at N = 2048, k = 200, 1e-13),
 // and one Chebyshev recurrence per pair serves all four series.
 // ---------------------------------------------------------------------------
-// J0, J1, G0, G1 at r for the node k; lkg = ln(k/2) + gamma
-static __device__ void je_values(cxd k, cxd lkg, double r, cxd& j0, cxd& j1, cxd& g0, cxd& g1) {
+// J0, J1, G0, G1 at r + dr for the node k; lkg = ln(k/2) + gamma. dr is what
+// the rounding of the panel point r left out: with the rounding of z = r k it is
+// a phase of up to 2^-53 |z|, which every pair of the panel would share, so the
+// values take it in to first order (|dz| < 1e-12).
+static __device__ void je_values(cxd k, cxd lkg, double r, double dr, cxd& j0, cxd& j1, cxd& g0, cxd& g1) {
   const double inv_pi = 0.31830988618379067154, two_over_pi = 0.63661977236758134308;
   if (r == 0.0) {
     j0 = cxd(1.0, 0.0);
@@ -1458,10 +1461,13 @@ static __device__ void je_values(cxd k, cxd lkg, double r, cxd& j0, cxd& j1, cxd
   } else {
     const Bessel01d b = bessel01(z);
     const double l = two_over_pi * log(r);
-    j0 = b.j0;
-    j1 = b.j1;
-    g0 = b.y0 - l * b.j0;
-    g1 = b.y1 - l * b.j1 + two_over_pi * cinv(z);
+    const cxd dz(fma(r, k.re, -z.re) + dr * k.re, fma(r, k.im, -z.im) + dr * k.im);
+    const cxd iz = cinv(z);
+    j0 = b.j0 - dz * b.j1;
+    j1 = b.j1 + dz * (b.j0 - iz * b.j1);
+    const cxd y0 = b.y0 - dz * b.y1, y1 = b.y1 + dz * (b.y0 - iz * b.y1);
+    g0 = y0 - l * j0;
+    g1 = y1 - l * j1 + two_over_pi * iz;
   }
 }
 
@@ -1492,15 +1498,16 @@ __global__ void __launch_bounds__(JE_BUILD_THREADS) k_cheb_build_je(ChebTables t
   const bool live = lp < ppb && p < t.nje;
   const cxd k = ks[q];
   if (live) {
-    const double a = (double)p * t.dr_je;
-    const double b = (p + 1 == t.nje) ? t.rmax : (double)(p + 1) * t.dr_je;
+    // the panel's ends and their sum are exact (make_cheb_je)
     const bool realk = (k.im == 0.0);
     const cxd kaL2 = 0.5 * cmul_i(k), kd = -0.5 * k;
     const cxd lkg = clog_d(0.5 * k) + cxd(0.57721566490153286061, 0.0);
     const double tn = cospi((double)n / (double)M);
-    const double r = 0.5 * ((b + a) + (b - a) * tn);
+    const double s = (double)(2 * p + 1) * t.dr_je, u = t.dr_je * tn;
+    const double r = 0.5 * (s + u);
+    const double dr = 0.5 * (u - (2.0 * r - s));  // |u| <= s: exact
     cxd j0, j1, g0, g1;
-    je_values(k, lkg, r, j0, j1, g0, g1);
+    je_values(k, lkg, r, dr, j0, j1, g0, g1);
     if (realk) { j0.im = 0.0; j1.im = 0.0; g0.im = 0.0; g1.im = 0.0; }
     fv[tid][0] = kaL2 * j1;
     fv[tid][1] = kaL2 * (j1 + cmul_i(g1));
@@ -1983,8 +1990,186 @@ __global__ void __launch_bounds__(256, 1) k_assemble_cheb_reduced_df(GeomDev g, 
   }
 }
 
-bool cheb_je_applies(const GeomDev& g, int deriv, int prec) {
-  return prec == QBG_PREC_MIXED && !deriv && g.m == g.n && g.quad != 1;
+// Symmetry-reduced DLP (value, complex64 forms) on the J/E tables, for orbits
+// of at most JR_MEM nodes with real scales. A reduced entry is the sum over the
+// members of its orbit of terms of the full operator's form,
+//   b U + i a P + kk  (je_fold), with the Kress split for the member I_b itself
+// and b = -c w_q sc, a = -b l, kk = b / (pi r) for an image, so every member is
+// one two-series evaluation and the table only resolves the oscillation (on the
+// H and J tables the near-r_min panels made the build the larger part).
+// CTA = 32 x 16 entries, a thread one entry's member per pass: per member the
+// tile's 512 distances are sorted by panel (so a warp reads few table rows), the
+// contributions go through shared memory by member, and a thread sums the
+// members of one entry and stores it, consecutive rows per warp.
+// Bound: the double-float recurrence's FP32 arithmetic and its row loads. Eight
+// disks of 24 nodes of the N = 4096 stadium reduced to m = 1024 (k near 300), from the
+// node assembly to the moments: 211 ms on the H and J tables, 157 ms here (60 ms of it
+// the assembly). Error against the FP64 direct assembly at those sizes, panels of
+// degree 9: rms 8.9e-15 (1.3e-14 on the H and J tables).
+constexpr int JR_MEM = 4, JR_T = 512;
+
+__global__ void __launch_bounds__(JR_T, 1) k_assemble_je_reduced(GeomDev g, ChebTables t, const cxd* __restrict__ ks, int nk,
+                                                                 void* const* __restrict__ outs,
+                                                                 void* const* __restrict__ los, long long ld) {
+  extern __shared__ float4 smem_jr[];
+  float4* stg = smem_jr;                                          // [2][JR_MEM][JR_T]
+  unsigned* keys = reinterpret_cast<unsigned*>(smem_jr);          // [JR_T], before the node loop
+  __shared__ int mem_q[JR_MEM][16];                               // member nodes of the tile's columns (-1: none)
+  __shared__ double mem_s[JR_MEM][16];                            // and their scales
+  const int tid = threadIdx.x;
+  const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 16;
+  const unsigned NOPANEL = (1u << 22) - 1;
+  // members of a column: I_b first, then its images
+  if (tid < 16) {
+    const int b = b0 + tid;
+    int c = 0;
+    for (int l = 0; l < JR_MEM; ++l) mem_q[l][tid] = -1;
+    if (b < g.m) {
+      const int j = g.fund[b];
+      mem_q[c++][tid] = j;
+      for (int l = 0; l < g.norb; ++l) {
+        const int q = g.orb[b * g.norb + l];
+        if (q == j || c >= JR_MEM) continue;
+        mem_s[c][tid] = g.orb_scale[2 * (b * g.norb + l)];
+        mem_q[c++][tid] = q;
+      }
+    }
+  }
+  __syncthreads();
+  int slot[JR_MEM], pan[JR_MEM];  // entry of the slot | tail degree << 10, table panel; slot < 0: none
+  dfl tt[JR_MEM], cb[JR_MEM], ca[JR_MEM];
+#pragma unroll
+  for (int l = 0; l < JR_MEM; ++l) {
+    {
+      const int a = a0 + (tid & 31), jl = tid >> 5, q = mem_q[l][jl];
+      unsigned pk = NOPANEL;
+      if (a < g.m && q >= 0) {
+        const int i = g.fund[a];
+        const float dx = (float)(g.x[i] - g.x[q]), dy = (float)(g.y[i] - g.y[q]);
+        int qp = (int)(sqrtf(fmaf(dx, dx, dy * dy)) * (float)t.invdr_je);
+        qp = qp < 0 ? 0 : (qp >= t.nje ? t.nje - 1 : qp);
+        if (i != q) pk = (unsigned)qp;
+      }
+      keys[tid] = (pk << 9) | (unsigned)tid;
+    }
+    __syncthreads();
+    for (int kk = 2; kk <= JR_T; kk <<= 1)
+      for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+        if (tid < JR_T / 2) {
+          const int lo = 2 * tid - (tid & (jj - 1)), hi = lo + jj;
+          const unsigned x = keys[lo], y = keys[hi];
+          if ((x > y) == ((lo & kk) == 0)) {
+            keys[lo] = y;
+            keys[hi] = x;
+          }
+        }
+        __syncthreads();
+      }
+    const unsigned key = keys[tid];
+    __syncthreads();
+    const int e = (int)(key & (JR_T - 1));
+    slot[l] = -1;
+    pan[l] = 0;
+    tt[l] = cb[l] = ca[l] = dfl{0.f, 0.f};
+    if ((key >> 9) != NOPANEL) {
+      const int i = g.fund[a0 + (e & 31)], q = mem_q[l][e >> 5];
+      Fold f{0.0, 0.0, 0.0, 0.0};
+      double r;
+      if (l == 0) {
+        const PairGeom p = pair_geom(g, i, q);
+        f = fold_of<0>(p);
+        r = p.r;
+      } else {
+        const double dxq = g.x[i] - g.x[q], dyq = g.y[i] - g.y[q];
+        r = hypot(dxq, dyq);
+        if (r >= 2.220446049250313e-16) {
+          f.B = (g.nx[q] * dxq + g.ny[q] * dyq) / r * g.speed[q] * g.ws[q] * mem_s[l][e >> 5];
+        }
+      }
+      if (r >= 2.220446049250313e-16) {
+        double td = 0.0;
+        panel_of(r, 0.0, t.rmax, t.dr_je, t.invdr_je, t.nje, pan[l], td);
+        const JeCoef c = je_coef<0>(f, 0.63661977236758134308 * log(r), 1.0 / r);
+        tt[l] = df_of(td);
+        cb[l] = c.b;
+        ca[l] = c.a;
+        slot[l] = e | (t.JEm[pan[l]] << 10);
+      }
+    }
+  }
+  // the entry this thread sums and stores, and its part that no node changes:
+  // the diagonal value and the 1/r terms
+  const int ea = a0 + (tid & 31), eb = b0 + (tid >> 5);
+  const bool live = ea < g.m && eb < g.m;
+  dfl cst{0.f, 0.f};
+  if (live) {
+    const int i = g.fund[ea];
+    double c = 0.0;
+    for (int l = 0; l < JR_MEM; ++l) {
+      const int q = mem_q[l][tid >> 5];
+      if (q < 0) continue;
+      if (l == 0 && q == i) {
+        c += 1.0 - g.ws[i] * g.kappa[i];
+        continue;
+      }
+      const double dxq = g.x[i] - g.x[q], dyq = g.y[i] - g.y[q], r = hypot(dxq, dyq);
+      if (q == i || r < 2.220446049250313e-16) continue;
+      double B;
+      if (l == 0) {
+        B = fold_of<0>(pair_geom(g, i, q)).B;
+      } else {
+        B = (g.nx[q] * dxq + g.ny[q] * dyq) / r * g.speed[q] * g.ws[q] * mem_s[l][tid >> 5];
+      }
+      c -= B * 0.31830988618379067154 / r;
+    }
+    cst = df_of(c);
+  }
+  // members without a term (the diagonal, none, coincident nodes) stay zero
+  for (int x = tid; x < 2 * JR_MEM * JR_T; x += JR_T) stg[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  const size_t off = (size_t)ea + (size_t)eb * (size_t)ld;
+  const int M = t.Mje;
+  for (int q = 0; q < nk; ++q) {
+    float4* s = stg + (q & 1) * JR_MEM * JR_T;
+#pragma unroll
+    for (int l = 0; l < JR_MEM; ++l)
+      if (slot[l] >= 0) {
+        dfl v[4];
+        je_series<2>(t.JE + ((size_t)q * t.nje + pan[l]) * (size_t)(M + 1) * 2, M, slot[l] >> 10, tt[l], v);
+        dfl re{0.f, 0.f}, im{0.f, 0.f};
+        df_acc(re, cb[l], v[2]);
+        df_acc(re, ca[l], v[1]);
+        df_acc(im, cb[l], v[3]);
+        df_acc(im, dfl{-ca[l].hi, -ca[l].lo}, v[0]);
+        s[l * JR_T + (slot[l] & 1023)] = make_float4(re.hi, re.lo, im.hi, im.lo);
+      }
+    __syncthreads();
+    if (live) {
+      dfl re = cst, im{0.f, 0.f};
+#pragma unroll
+      for (int l = 0; l < JR_MEM; ++l) {
+        const float4 v = s[l * JR_T + tid];
+        const dfl x = df_two_sum(re.hi, v.x), y = df_two_sum(im.hi, v.z);
+        re = dfl{x.hi, re.lo + (x.lo + v.y)};
+        im = dfl{y.hi, im.lo + (y.lo + v.w)};
+      }
+      re = df_norm(re);
+      im = df_norm(im);
+      reinterpret_cast<cxf*>(outs[q])[off] = cxf(re.hi, im.hi);
+      if (los) reinterpret_cast<cxf*>(los[q])[off] = cxf(re.lo, im.lo);
+    }
+  }
+}
+
+// Reduced operators only with panels of degree 7 and more, as the tuners choose
+// them: there both interpolants agree to the panels' tolerance. With the
+// reference's default degree 5 they differ by the H panels' own error, 3e-12 to
+// 6e-12 of an entry of 1e-3 max|A| at k = 30, and the mixed form stays on the
+// tables of the FP64 form.
+bool cheb_je_applies(const GeomDev& g, int deriv, int prec, const qbg_cheb_params& prm) {
+  if (prec != QBG_PREC_MIXED || deriv || g.quad == 1) return false;
+  if (g.m == g.n) return true;
+  return g.form == 0 && g.norb <= JR_MEM && g.orb_real && prm.M_h >= 7 && prm.M_j >= 7;
 }
 
 size_t cheb_je_bytes(const ChebTables& t) {
@@ -2155,6 +2340,11 @@ int launch_assemble_cheb(const GeomDev& g, const ChebTables& t, const cxd* ks, i
         k_assemble_cheb_reduced<1, 0><<<grd, blk, 0, st>>>(g, t, ks, nk, kchunk, outs_dev, nullptr, ld);
       else
         k_assemble_cheb_reduced<0, 0><<<grd, blk, 0, st>>>(g, t, ks, nk, kchunk, outs_dev, nullptr, ld);
+    } else if (t.JE && prec == QBG_PREC_MIXED) {
+      const int dyn = (int)sizeof(float4) * 2 * JR_MEM * JR_T;
+      QBG_CUDA(cudaFuncSetAttribute(k_assemble_je_reduced, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+      k_assemble_je_reduced<<<dim3((g.m + 31) / 32, (g.m + 15) / 16), JR_T, dyn, st>>>(g, t, ks, nk, outs_dev, lo_outs_dev,
+                                                                                      ld);
     } else if (t.HD && t.JD && t.nkc && g.norb <= 4) {
       dim3 dgrd((g.m + 31) / 32, (g.m + 7) / 8, 1);
       const int dm = (t.Mh == t.Mj) ? t.Mh : 0;

@@ -54,9 +54,9 @@ int cheb_build(ChebTables& t, const cxd* ks, cudaStream_t st);
 // sizes cheb_df_bytes reports, owned by the caller); after cheb_build
 void cheb_df_bytes(const ChebTables& t, size_t* hd, size_t* jd, size_t* nkc);
 int cheb_df_tables(ChebTables& t, const cxd* ks, cudaStream_t st);
-// the J/E tables of the mixed form's full symmetric assembly: whether they
-// apply, their bytes (t.nk, nje, Mje, nse set), and their build (t.JE set)
-bool cheb_je_applies(const GeomDev& g, int deriv, int prec);
+// the J/E tables of the mixed form's assembly of full operators and of the DLP
+// reduced by reflections: whether they apply with these panels, their bytes (t.nk, nje, Mje, nse set), and their build (t.JE set)
+bool cheb_je_applies(const GeomDev& g, int deriv, int prec, const qbg_cheb_params& prm);
 size_t cheb_je_bytes(const ChebTables& t);
 int cheb_je_build(ChebTables& t, const cxd* ks, cudaStream_t st);
 // whether the complex64 Chebyshev assembly of g runs on double-float tables

@@ -215,7 +215,7 @@ int load(qbg_beyn* b, int n0, int c) {
     std::vector<void*> ctmp;
     ChebTables t;
     int s = QBG_OK;
-    if (cheb_je_applies(b->g->d, 0, b->prec)) {
+    if (cheb_je_applies(b->g->d, 0, b->prec, cp)) {
       s = make_cheb_je(b->g, b->zj + n0, c, cp, t, ctmp, st);
     } else {
       s = make_cheb(b->g, b->zj + n0, c, cp, t, ctmp, st);

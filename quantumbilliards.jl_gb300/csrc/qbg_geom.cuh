@@ -33,6 +33,7 @@ struct GeomDev {
   const int* fund = nullptr;      // m: full index of fundamental node a
   const int* orb = nullptr;       // m*norb: images q of fundamental node b
   const double* orb_scale = nullptr;  // m*norb complex (re, im) scale factors
+  int orb_real = 0;               // every scale factor is real (reflections)
   const double* nx = nullptr;     // unit normals (ty, -tx)/|t| for image terms
   const double* ny = nullptr;
   // Alpert quadrature (quad == 1)
