@@ -13,17 +13,17 @@
 // D += A_big B_big + A_big B_small + A_small B_big (the dropped small*small
 // term is ~2^-22 relative).
 //
-// One CTA (128 threads) computes a 128 x 32 complex tile (real 128 x 64,
-// tcgen05.mma.cta_group::1.kind::tf32 with M = 128, N = 64, K = 8). Threads
-// stage the operands in shared memory in the canonical K-major layout without
+// One CTA (16 staging warps and one that issues) computes a 128 x 32 complex tile
+// (real 128 x 64, tcgen05.mma.cta_group::1.kind::tf32, K = 8). The staging warps
+// write the operands to shared memory in the canonical K-major layout without
 // swizzle (8-row x 16-byte core matrices; LBO = 128 B between the two core
-// matrices along K, SBO = 256 B between 8-row groups) with 16-byte stores, in
-// two stages of 16 complex k (48 KB each, two CTAs per SM); thread 0 issues
-// the MMAs and commits each stage to its own mbarrier; the accumulator lives in
-// 64 TMEM columns and is read back with tcgen05.ld.32x32b. C is fetched into
-// registers before the k loop. Every mbarrier wait is
-// bounded: on timeout the kernel records an error, waits (bounded) for its own
-// MMAs, frees its TMEM and returns without writing C.
+// matrices along K, SBO = 256 B between 8-row groups), in two stages of 16
+// complex k (48 KB each, two CTAs per SM); lane 0 of the last warp issues the
+// MMAs and commits each stage to its own mbarrier; the accumulators live in
+// 128 TMEM columns and are read back with tcgen05.ld.32x32b. C is fetched into
+// registers before the k loop. Every mbarrier wait is bounded: on timeout the
+// kernel records an error, waits (bounded) for its own MMAs, frees its TMEM and
+// returns without writing C.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -45,19 +45,24 @@ constexpr int TC_KSTEPS = 4;
 constexpr int TC_A_STEP = TC_BM * 8;        // floats per operand block per MMA step (4 KB)
 constexpr int TC_B_STEP = 2 * TC_BN * 8;    // floats (2 KB)
 constexpr int TC_STAGE_FLOATS = 2 * TC_KSTEPS * (TC_A_STEP + TC_B_STEP);  // big + small, A and B (48 KB)
-constexpr uint32_t TC_TMEM_COLS = 64;
+constexpr uint32_t TC_TMEM_COLS = 128, PK_TMEM_COLS = 64;
 constexpr long long TC_SPIN_LIMIT = 1ll << 26;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-
-__device__ __forceinline__ float tf32_rna(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
+// x = big + small + O(2^-23 |x|), both rounded to tf32 (nearest, ties away from zero)
+// on the integer unit: the conversion instruction's throughput showed as a stall of the
+// staging warps (0.84 of 8.4 cycles an instruction, 0.65 so). A NaN leaves big finite
+// (0x7fffffff wraps to -0) and stays in small, whose rounding is applied as a
+// floating-point correction (exact: r - s is the rounding error of s); an
+// infinity gives big = inf, small = NaN.
+__device__ __forceinline__ void tf32_split(float x, float& big, float& small) {
+  big = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  const float s = x - big;
+  const float r = __uint_as_float((__float_as_uint(s) + 0x1000u) & 0xffffe000u);
+  small = s + (r - s);
 }
-
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
   const uint64_t lbo = 128, sbo = 256;
@@ -70,12 +75,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 
 // instruction descriptor: D f32, A/B tf32, both K-major, N = 64, M = 128
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t TC_IDESC2 = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);  // N = 128
 
-__device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t da, uint64_t db, uint32_t acc) {
+__device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
-      "l"(da), "l"(db), "r"(TC_IDESC), "r"(acc));
+      "l"(da), "l"(db), "r"(idesc), "r"(acc));
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
@@ -100,8 +106,9 @@ __device__ long long g_tc_wait_polls = TC_SPIN_LIMIT;
 // bounded wait: gives up after ~0.5 s of SM clock (1e9 cycles) or `polls` polls
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity,
                                                   long long polls = TC_SPIN_LIMIT) {
+  if (polls > 0 && mbar_try(mbar, parity)) return true;
   const long long t0 = clock64();
-  for (long long it = 0; it < polls; ++it) {
+  for (long long it = 1; it < polls; ++it) {
     if (mbar_try(mbar, parity)) return true;
     if (clock64() - t0 > 1000000000ll) break;
   }
@@ -109,31 +116,38 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t mbar, uint32_t parity
 }
 
 
-// Operand staging. A tile: thread = row i, 16 complex k of one k-tile, held in
-// registers between the global load and the shared-memory store so that the
-// loads of tile kt+1 are in flight while the tensor cores work on tile kt.
+// Operand staging by TC_T = 512 threads: each holds 4 complex k of one row of
+// the A tile (one MMA step) and one element of the B tile in registers between
+// the global load and the shared-memory store. A warp's B elements are 4
+// consecutive k of 8 columns (whole 32-byte sectors; with the lane order below
+// each half-warp's 8-byte store covers 128 consecutive bytes).
+constexpr int TC_T = 512;
 struct TcRegs {
-  cxf a[TC_BK];   // A(m0 + tid, k0 + kc)
-  cxf b[2][2];    // B(k0 + 2p + {0,1}, n0 + j) for the two (p, j) items of this thread
+  cxf a[4];  // A(m0 + row, k0 + 4 grp + q)
+  cxf b;     // B(k0 + bk, n0 + bj)
+};
+struct TcPos {
+  int row, grp, bk, bj;
 };
 
-__device__ __forceinline__ void tc_load(TcRegs& r, const cxf* __restrict__ Ab, long long lda, const cxf* __restrict__ Bb,
-                                        long long ldb, int M, int N, int K, int m0, int n0, int k0, int tid) {
-  const int gi = m0 + tid;
-  const bool rowok = gi < M;
+__device__ __forceinline__ TcPos tc_pos(int tid) {
+  const int lane = tid & 31, warp = tid >> 5;
+  return TcPos{tid & 127, tid >> 7, 4 * (warp & 3) + 2 * (lane >> 4) + (lane & 1), 8 * (warp >> 2) + ((lane >> 1) & 7)};
+}
+
+// pa, pb: this thread's first A and its B element of the tile; kleft = K - k0.
+// Rows past M and columns past N repeat the last one (their results are not
+// stored); k past K are zeros.
+__device__ __forceinline__ void tc_load(TcRegs& r, const TcPos& t, const cxf* __restrict__ pa, long long lda,
+                                        const cxf* pb, int kleft) {
+  if (kleft >= TC_BK) {
 #pragma unroll
-  for (int kc = 0; kc < TC_BK; ++kc) {
-    const int gk = k0 + kc;
-    r.a[kc] = (rowok && gk < K) ? Ab[(long long)gi + (long long)gk * lda] : cxf(0.f, 0.f);
-  }
+    for (int q = 0; q < 4; ++q) r.a[q] = pa[q * lda];
+    r.b = *pb;
+  } else {
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int item = tid + 128 * q;
-    const int j = item & (TC_BN - 1), p = item >> 5;  // j fastest: conflict-free shared stores
-    const int gj = n0 + j, gk = k0 + 2 * p;
-    const bool colok = gj < N;
-    r.b[q][0] = (colok && gk < K) ? Bb[(long long)gk + (long long)gj * ldb] : cxf(0.f, 0.f);
-    r.b[q][1] = (colok && gk + 1 < K) ? Bb[(long long)(gk + 1) + (long long)gj * ldb] : cxf(0.f, 0.f);
+    for (int q = 0; q < 4; ++q) r.a[q] = 4 * t.grp + q < kleft ? pa[q * lda] : cxf(0.f, 0.f);
+    r.b = t.bk < kleft ? *pb : cxf(0.f, 0.f);
   }
 }
 
@@ -141,182 +155,183 @@ __device__ __forceinline__ void tc_load(TcRegs& r, const cxf* __restrict__ Ab, l
 __device__ __forceinline__ int kmaj4(int row, int c) { return (row >> 3) * 64 + c * 32 + (row & 7) * 4; }
 
 __device__ __forceinline__ void split4(float x0, float x1, float x2, float x3, float4& big, float4& small) {
-  big = make_float4(tf32_rna(x0), tf32_rna(x1), tf32_rna(x2), tf32_rna(x3));
-  small = make_float4(tf32_rna(x0 - big.x), tf32_rna(x1 - big.y), tf32_rna(x2 - big.z), tf32_rna(x3 - big.w));
+  tf32_split(x0, big.x, small.x);
+  tf32_split(x1, big.y, small.y);
+  tf32_split(x2, big.z, small.z);
+  tf32_split(x3, big.w, small.w);
 }
 
-__device__ __forceinline__ void tc_store(const TcRegs& r, float* sAb, float* sAs, float* sBb, float* sBs, int tid) {
-  // A'[i][2k] = Re, A'[i][2k+1] = Im; pair p = complex k 2p, 2p+1 -> MMA step p/2, 16-byte segment p%2
+__device__ __forceinline__ void tc_store(const TcRegs& r, const TcPos& t, float* sAb, float* sAs, float* sB) {
+  // A'[i][2k] = Re, A'[i][2k+1] = Im; pair p of the step's complex k is its 16-byte segment p
 #pragma unroll
-  for (int p = 0; p < TC_BK / 2; ++p) {
+  for (int p = 0; p < 2; ++p) {
     float4 big, small;
     split4(r.a[2 * p].re, r.a[2 * p].im, r.a[2 * p + 1].re, r.a[2 * p + 1].im, big, small);
-    const int off = (p >> 1) * TC_A_STEP + kmaj4(tid, p & 1);
+    const int off = t.grp * TC_A_STEP + kmaj4(t.row, p);
     *reinterpret_cast<float4*>(sAb + off) = big;
     *reinterpret_cast<float4*>(sAs + off) = small;
   }
   // B'[j] = (Re, -Im) and B'[BN + j] = (Im, Re) along k
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int item = tid + 128 * q;
-    const int j = item & (TC_BN - 1), p = item >> 5;
-    const cxf v0 = r.b[q][0], v1 = r.b[q][1];
-    float4 big, small;
-    const int base = (p >> 1) * TC_B_STEP;
-    split4(v0.re, -v0.im, v1.re, -v1.im, big, small);
-    *reinterpret_cast<float4*>(sBb + base + kmaj4(j, p & 1)) = big;
-    *reinterpret_cast<float4*>(sBs + base + kmaj4(j, p & 1)) = small;
-    split4(v0.im, v0.re, v1.im, v1.re, big, small);
-    *reinterpret_cast<float4*>(sBb + base + kmaj4(TC_BN + j, p & 1)) = big;
-    *reinterpret_cast<float4*>(sBs + base + kmaj4(TC_BN + j, p & 1)) = small;
-  }
+  float br, bi, sr, si;
+  tf32_split(r.b.re, br, sr);
+  tf32_split(r.b.im, bi, si);
+  const int lo = (t.bk >> 2) * 2 * TC_B_STEP + 2 * (t.bk & 1), seg = (t.bk >> 1) & 1;
+  const int o0 = lo + kmaj4(t.bj, seg), o1 = lo + kmaj4(TC_BN + t.bj, seg);
+  *reinterpret_cast<float2*>(sB + o0) = make_float2(br, -bi);
+  *reinterpret_cast<float2*>(sB + TC_B_STEP + o0) = make_float2(sr, -si);
+  *reinterpret_cast<float2*>(sB + o1) = make_float2(bi, br);
+  *reinterpret_cast<float2*>(sB + TC_B_STEP + o1) = make_float2(si, sr);
 }
 
 }  // namespace
 
-// Two shared-memory stages: while the tensor cores read stage kt&1, the
-// threads hold tile kt+1 in registers and then store it into the other stage
-// once the MMAs of tile kt-1 (which read that stage) have been observed done.
-__global__ void __launch_bounds__(128) k_tc_cgemm(int M, int N, int K, cxf alpha, const cxf* __restrict__ A,
-                                                  long long lda, long long sA, const cxf* B, long long ldb,
-                                                  long long sB, cxf beta, cxf* C, long long ldc, long long sC,
-                                                  int batch2, long long sA2, long long sB2, long long sC2,
-                                                  int* err) {
+// Warps 0..15 stage the operands, warp 16 issues the MMAs: while the tensor cores
+// read one of the two shared-memory stages, the others store the next tile, and
+// the loads of the two tiles after it are in flight in registers. full[s] counts
+// the staging warps, empty[s] completes with the MMAs that read stage s.
+// The two products of A_big, with B_big and with B_small, are one MMA of N = 128
+// (B' = [big | small] of a step, an N = 64 MMA takes no less time); A_small B_big
+// joins the columns of A_big B_small, and the epilogue adds the two halves.
+// Bound at the solves' sizes (K = 256, few tiles): the chain of one k-tile, load,
+// split, store and MMA. A product of 256 x 96 x 256 for 10 operators takes 16.5 us
+// (128 threads that also issued three N = 64 MMAs a step: 25 us); one disk of 48
+// nodes of N = 2048: 60.7 -> 56.9 ms, 16 streamed nodes of N = 5002: 165.5 -> 152 ms.
+__global__ void __launch_bounds__(TC_T + 32, 2) k_tc_cgemm(int M, int N, int K, cxf alpha, const cxf* __restrict__ A,
+                                                           long long lda, long long sA, const cxf* B, long long ldb,
+                                                           long long sB, cxf beta, cxf* C, long long ldc,
+                                                           long long sC, int batch2, long long sA2, long long sB2,
+                                                           long long sC2, int* err) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
-  float* stage_base = reinterpret_cast<float*>(tc_smem);  // [2][sAb | sAs | sBb | sBs]
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(stage_base + 2 * TC_STAGE_FLOATS);  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 2);
+  float* stage_base = reinterpret_cast<float*>(tc_smem);  // [2][sAb | sAs | sB]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(stage_base + 2 * TC_STAGE_FLOATS);  // full[2], empty[2], done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 5);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool stager = warp < TC_T / 32;
   const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TC_BN;
   const long long bo = blockIdx.z / batch2, bi = blockIdx.z % batch2;  // outer, inner batch index
   const cxf* Ab = A + bo * sA + bi * sA2;
   const cxf* Bb = B + bo * sB + bi * sB2;
   cxf* Cb = C + bo * sC + bi * sC2;
 
-  if (warp == 0) {
+  if (!stager) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TC_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  const uint32_t mb = smem_u32(mbar);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + 1)) : "memory");
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb + 8 * q), "r"(q < 2 ? TC_T / 32 : 1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *abort_flag = (*reinterpret_cast<volatile int*>(err) != 0) ? 1 : 0;
   }
-
-  // C of this thread's row, fetched now so that its latency hides behind the k loop
-  const int i = m0 + warp * 32 + lane;  // TMEM lane = row within the tile = tid
-  const bool use_beta = !(beta.re == 0.f && beta.im == 0.f);
-  cxf cold[TC_BN];
-#pragma unroll
-  for (int j = 0; j < TC_BN; ++j) {
-    const int gj = n0 + j;
-    cold[j] = (use_beta && i < M && gj < N) ? Cb[(long long)i + (long long)gj * ldc] : cxf(0.f, 0.f);
+  const TcPos pos = tc_pos(tid & (TC_T - 1));
+  const int ktiles = (K + TC_BK - 1) / TC_BK;
+  TcRegs regs[2];
+  const cxf* pa = Ab + min(m0 + pos.row, M - 1) + (long long)(4 * pos.grp) * lda;
+  const cxf* pb = Bb + pos.bk + (long long)min(n0 + pos.bj, N - 1) * ldb;
+  const long long step = TC_BK * lda;
+  if (stager) {
+    tc_load(regs[0], pos, pa, lda, pb, K);
+    tc_load(regs[1], pos, pa += step, lda, pb += TC_BK, K - TC_BK);
   }
-
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t mb0 = smem_u32(mbar), mb1 = smem_u32(mbar + 1);
-  // per stage: parity of the next completion of its barrier, and whether a
-  // commit to it has not been observed complete yet (uniform over the CTA)
-  uint32_t wph0 = 0u, wph1 = 0u;
-  bool pend0 = false, pend1 = false;
-  const int ktiles = (K + TC_BK - 1) / TC_BK;
-  bool ok = (*abort_flag == 0);
+  const bool go = *abort_flag == 0;
 
-  TcRegs regs;
-  if (ok && ktiles > 0) tc_load(regs, Ab, lda, Bb, ldb, M, N, K, m0, n0, 0, tid);
-  for (int kt = 0; kt < ktiles && ok; ++kt) {
-    const int st = kt & 1;
-    float* sAb = stage_base + st * TC_STAGE_FLOATS;
-    float* sAs = sAb + TC_KSTEPS * TC_A_STEP;
-    float* sBb = sAs + TC_KSTEPS * TC_A_STEP;
-    float* sBs = sBb + TC_KSTEPS * TC_B_STEP;
-    if (st ? pend1 : pend0) {
-      // the MMAs of tile kt-2 read this stage
-      if (mbar_wait_bounded(st ? mb1 : mb0, st ? wph1 : wph0, g_tc_wait_polls)) {
-        if (st) { wph1 ^= 1u; pend1 = false; } else { wph0 ^= 1u; pend0 = false; }
-      } else {
-        atomicExch(abort_flag, 1);
+  // C of this thread (row = TMEM lane tid & 127, 8 of the tile's columns), fetched now so that its
+  // latency hides behind the k loop
+  const int i = m0 + pos.row, jc = n0 + 8 * pos.grp;
+  const bool use_beta = !(beta.re == 0.f && beta.im == 0.f);
+  cxf cold[8];
+  if (stager && go) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      cold[j] = (use_beta && i < M && jc + j < N) ? Cb[(long long)i + (long long)(jc + j) * ldc] : cxf(0.f, 0.f);
+#pragma unroll 2
+    for (int kt = 0; kt < ktiles; ++kt) {
+      const int st = kt & 1;
+      float* sAb = stage_base + st * TC_STAGE_FLOATS;
+      float* sAs = sAb + TC_KSTEPS * TC_A_STEP;
+      float* sBt = sAs + TC_KSTEPS * TC_A_STEP;
+      if (kt >= 2 && !mbar_wait_bounded(mb + 16 + 8 * st, (uint32_t)(((kt >> 1) - 1) & 1), g_tc_wait_polls)) {
+        atomicExch(abort_flag, 1);  // the MMAs of tile kt-2 still read this stage
+        break;
+      }
+      tc_store(st ? regs[1] : regs[0], pos, sAb, sAs, sBt);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mb + 8 * st) : "memory");
+      if (kt + 2 < ktiles) {
+        pa += step;
+        pb += TC_BK;
+        if (st) tc_load(regs[1], pos, pa, lda, pb, K - (kt + 2) * TC_BK);
+        else tc_load(regs[0], pos, pa, lda, pb, K - (kt + 2) * TC_BK);
       }
     }
-    tc_store(regs, sAb, sAs, sBb, sBs, tid);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (*abort_flag) {
-      ok = false;
-      break;
-    }
-    if (kt + 1 < ktiles) tc_load(regs, Ab, lda, Bb, ldb, M, N, K, m0, n0, (kt + 1) * TC_BK, tid);
-    if (tid == 0) {
+  } else if (!stager && lane == 0) {
+    int kt = 0;
+    for (; kt < ktiles && go; ++kt) {
+      const int st = kt & 1;
+      const uint32_t sAb = smem_u32(stage_base + st * TC_STAGE_FLOATS);
+      const uint32_t sAs = sAb + 4 * TC_KSTEPS * TC_A_STEP, sBt = sAs + 4 * TC_KSTEPS * TC_A_STEP;
+      if (!mbar_wait_bounded(mb + 8 * st, (uint32_t)((kt >> 1) & 1), g_tc_wait_polls)) {
+        atomicExch(abort_flag, 1);
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int s = 0; s < TC_KSTEPS; ++s) {
-        const uint64_t dab = smem_desc(smem_u32(sAb + s * TC_A_STEP));
-        const uint64_t das = smem_desc(smem_u32(sAs + s * TC_A_STEP));
-        const uint64_t dbb = smem_desc(smem_u32(sBb + s * TC_B_STEP));
-        const uint64_t dbs = smem_desc(smem_u32(sBs + s * TC_B_STEP));
-        mma_tf32(tmem, das, dbb, (kt | s) != 0);
-        mma_tf32(tmem, dab, dbs, 1);
-        mma_tf32(tmem, dab, dbb, 1);
+        const uint64_t dab = smem_desc(sAb + 4 * s * TC_A_STEP), das = smem_desc(sAs + 4 * s * TC_A_STEP);
+        const uint64_t db = smem_desc(sBt + 8 * s * TC_B_STEP);
+        mma_tf32(tmem, dab, db, TC_IDESC2, (kt | s) != 0);
+        mma_tf32(tmem + 2 * TC_BN, das, db, TC_IDESC, 1);
       }
-      mma_commit(st ? mb1 : mb0);
+      mma_commit(mb + 16 + 8 * st);
     }
-    if (st) pend1 = true; else pend0 = true;
+    // every MMA issued must be observed done before TMEM is read or released
+    mma_commit(mb + 32);
+    if (!mbar_wait_bounded(mb + 32, 0)) atomicExch(abort_flag, 1);
   }
-  // drain: every committed group must be observed before TMEM is read or released
-  bool drained = true;
-  if (pend0 && !mbar_wait_bounded(mb0, wph0)) drained = false;
-  if (pend1 && !mbar_wait_bounded(mb1, wph1)) drained = false;
-  if (!drained) atomicExch(abort_flag, 1);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (*abort_flag || ktiles == 0) {
     if (tid == 0 && *abort_flag) atomicExch(err, 1);
-  } else {
-    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-    uint32_t re[32], im[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(re[0]), "=r"(re[1]), "=r"(re[2]), "=r"(re[3]), "=r"(re[4]), "=r"(re[5]), "=r"(re[6]), "=r"(re[7]),
-          "=r"(re[8]), "=r"(re[9]), "=r"(re[10]), "=r"(re[11]), "=r"(re[12]), "=r"(re[13]), "=r"(re[14]),
-          "=r"(re[15]), "=r"(re[16]), "=r"(re[17]), "=r"(re[18]), "=r"(re[19]), "=r"(re[20]), "=r"(re[21]),
-          "=r"(re[22]), "=r"(re[23]), "=r"(re[24]), "=r"(re[25]), "=r"(re[26]), "=r"(re[27]), "=r"(re[28]),
-          "=r"(re[29]), "=r"(re[30]), "=r"(re[31])
-        : "r"(taddr));
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(im[0]), "=r"(im[1]), "=r"(im[2]), "=r"(im[3]), "=r"(im[4]), "=r"(im[5]), "=r"(im[6]), "=r"(im[7]),
-          "=r"(im[8]), "=r"(im[9]), "=r"(im[10]), "=r"(im[11]), "=r"(im[12]), "=r"(im[13]), "=r"(im[14]),
-          "=r"(im[15]), "=r"(im[16]), "=r"(im[17]), "=r"(im[18]), "=r"(im[19]), "=r"(im[20]), "=r"(im[21]),
-          "=r"(im[22]), "=r"(im[23]), "=r"(im[24]), "=r"(im[25]), "=r"(im[26]), "=r"(im[27]), "=r"(im[28]),
-          "=r"(im[29]), "=r"(im[30]), "=r"(im[31])
-        : "r"(taddr + (uint32_t)TC_BN));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  } else if (stager) {
+    // warp w reads TMEM lanes 32 (w mod 4) .., columns 8 grp .. of Re and Im of both halves
+    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(8 * pos.grp);
+    float v[4][8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t x[8];
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
+                   : "r"(taddr + (uint32_t)(q * TC_BN)));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[q][j] = __uint_as_float(x[j]);
+    }
     if (i < M) {
 #pragma unroll
-      for (int j = 0; j < TC_BN; ++j) {
-        const int gj = n0 + j;
-        if (gj < N) {
-          cxf v = alpha * cxf(__uint_as_float(re[j]), __uint_as_float(im[j]));
-          if (use_beta) v += beta * cold[j];
-          Cb[(long long)i + (long long)gj * ldc] = v;
+      for (int j = 0; j < 8; ++j) {
+        if (jc + j < N) {
+          cxf c = alpha * cxf(v[0][j] + v[2][j], v[1][j] + v[3][j]);
+          if (use_beta) c += beta * cold[j];
+          Cb[(long long)i + (long long)(jc + j) * ldc] = c;
         }
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
+  if (!stager) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
   }
@@ -425,7 +440,7 @@ __global__ void __launch_bounds__(128, 1) k_tc_cgemm_pk(int M, int N, int KT, cx
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TC_TMEM_COLS)
+                 "r"(PK_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -486,9 +501,9 @@ __global__ void __launch_bounds__(128, 1) k_tc_cgemm_pk(int M, int N, int KT, cx
         const uint64_t das = smem_desc(smem_u32(sA + TC_KSTEPS * TC_A_STEP + q * TC_A_STEP));
         const uint64_t dbb = smem_desc(smem_u32(sB + q * TC_B_STEP));
         const uint64_t dbs = smem_desc(smem_u32(sB + TC_KSTEPS * TC_B_STEP + q * TC_B_STEP));
-        mma_tf32(tmem, das, dbb, (kt | q) != 0);
-        mma_tf32(tmem, dab, dbs, 1);
-        mma_tf32(tmem, dab, dbb, 1);
+        mma_tf32(tmem, das, dbb, TC_IDESC, (kt | q) != 0);
+        mma_tf32(tmem, dab, dbs, TC_IDESC, 1);
+        mma_tf32(tmem, dab, dbb, TC_IDESC, 1);
       }
       mma_commit(smem_u32(empty + s));
       ++committed;
@@ -559,7 +574,7 @@ __global__ void __launch_bounds__(128, 1) k_tc_cgemm_pk(int M, int N, int KT, cx
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PK_TMEM_COLS) : "memory");
   }
 }
 
@@ -981,7 +996,7 @@ int tc_gemm_c64(int M, int N, int K, cxf alpha, const cxf* A, long long lda, lon
     return QBG_OK;
   }
   dim3 grd(MT, NT, nb);
-  k_tc_cgemm<<<grd, 128, tc_smem_bytes(), st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch2,
+  k_tc_cgemm<<<grd, TC_T + 32, tc_smem_bytes(), st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch2,
                                                  sA2, sB2, sC2, derr);
   QBG_LAUNCH_CHECK("k_tc_cgemm");
   return QBG_OK;
