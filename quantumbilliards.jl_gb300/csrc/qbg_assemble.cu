@@ -1471,87 +1471,174 @@ static __device__ void je_values(cxd k, cxd lkg, double r, double dr, cxd& j0, c
   }
 }
 
-// CTA = (JE_BUILD_THREADS / (M + 1)) panels of one node, one thread per
-// Chebyshev-Lobatto point (the FP64 Bessel evaluation is the cost: one
-// thread per panel left the FP64 pipe idle on latency); then one thread per
-// (panel, degree) forms the DCT-I coefficients (as k_cheb_build) from the
-// values in shared memory and stores their double-float split; last, one
-// thread per panel folds the panel's FP32-tail degree into JEm by atomicMax
-// (the largest over the nodes, so the assembly reads it once per pair).
-constexpr int JE_BUILD_THREADS = 128;
+// t^n = sum_m c[n][m] T_m(t): c = 2^{1-n} binom(n, (n - m) / 2), halved at m = 0,
+// for m <= n of n's parity
+constexpr int JE_NT = 24;
+struct TaylorToCheb {
+  double c[JE_NT][QBG_CHEB_MAX_DEGREE + 1];
+};
+constexpr TaylorToCheb taylor_to_cheb() {
+  TaylorToCheb t{};
+  for (int n = 0; n < JE_NT; ++n) {
+    double b = 1.0;
+    for (int i = 0; i < n; ++i) b *= 0.5;  // 2^-n binom(n, j), j = (n - m) / 2
+    for (int j = 0; 2 * j <= n; ++j) {
+      const int m = n - 2 * j;
+      if (m <= QBG_CHEB_MAX_DEGREE) t.c[n][m] = m == 0 ? b : 2.0 * b;
+      b = b * (n - j) / (j + 1);
+    }
+  }
+  return t;
+}
+static __device__ const TaylorToCheb g_taylor_to_cheb = taylor_to_cheb();
+
+// CTA = 32 panels of one node. Bound: FP64 instructions (the pipe was 75-79%
+// busy when every Chebyshev-Lobatto point of a panel took its own Bessel
+// evaluation). One evaluation at the panel's centre gives the Taylor series in
+// t = (r - centre) / h of all four functions, from their equations
+//   J0' = -J1, z J1' = z J0 - J1,
+//   z G0' = -z G1 + (2/pi)(1 - J0), z G1' = z G0 - G1 - (2/pi) J1
+// with z = z0 + w t (a lane a panel), and a second pass turns it into Chebyshev
+// coefficients (lane = panel, degrees over the warps), stored as their
+// double-float split. 24 terms reach 1e-19 for |w| <= 1.5, and from the panel
+// at 4.5 widths on |w / z0| <= 1/9, so the division by z0 in the recurrences
+// amplifies nothing. The panels before it, and all panels of a node with wider
+// ones, are sampled at the Lobatto points and transformed (DCT-I). Last, a lane
+// a panel folds its FP32-tail degree into JEm by atomicMax (the largest over
+// the nodes, so the assembly reads it once per pair).
+// 384 nodes, 3400 panels, two series: 14.7 -> 4.9 ms; 16 nodes, 4500 panels of
+// degree 5, four series: 0.67 -> 0.28 ms.
+constexpr int JE_BUILD_THREADS = 128, JE_PPC = 32, JE_NEAR = 4;
+
+template <int NS>
+__host__ __device__ constexpr size_t je_build_smem(int M) {
+  return sizeof(cxd) * JE_NT * NS * JE_PPC + sizeof(float) * (M + 1) * NS * JE_PPC + sizeof(double) * (M + 1) * (M + 1);
+}
 
 template <int NS>
 __global__ void __launch_bounds__(JE_BUILD_THREADS) k_cheb_build_je(ChebTables t, const cxd* __restrict__ ks) {
-  constexpr int MMAX = QBG_CHEB_MAX_DEGREE;
-  __shared__ cxd fv[JE_BUILD_THREADS][NS];
-  __shared__ double mag[JE_BUILD_THREADS][NS];
-  __shared__ double dct[(MMAX + 1) * (MMAX + 1)];
-  const int M = t.Mje, P = M + 1, ppb = JE_BUILD_THREADS / P;
-  const int q = blockIdx.y;
-  const int tid = threadIdx.x;
-  for (int x = tid; x < P * P; x += JE_BUILD_THREADS) {
-    const int jn = x / P, m = x % P;
-    dct[x] = cospi((double)(jn * m) / (double)M);  // cos(pi jn m / M)
-  }
-  const int lp = tid / P, n = tid % P;
-  const int p = blockIdx.x * ppb + lp;
-  const bool live = lp < ppb && p < t.nje;
+  extern __shared__ cxd sm_je[];
+  cxd* fv = sm_je;  // [row][series][panel]: Taylor terms, or values at the Lobatto points (M + 1 <= JE_NT)
+  float* mag = reinterpret_cast<float*>(fv + JE_NT * NS * JE_PPC);          // [degree][series][panel]
+  double* dct = reinterpret_cast<double*>(mag + (t.Mje + 1) * NS * JE_PPC);  // cos(pi jn m / M)
+  const double two_over_pi = 0.63661977236758134308;
+  const int M = t.Mje, P = M + 1;
+  const int q = blockIdx.y, p0 = blockIdx.x * JE_PPC;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int np = min(JE_PPC, t.nje - p0);
   const cxd k = ks[q];
-  if (live) {
-    // the panel's ends and their sum are exact (make_cheb_je)
-    const bool realk = (k.im == 0.0);
-    const cxd kaL2 = 0.5 * cmul_i(k), kd = -0.5 * k;
+  const bool realk = (k.im == 0.0);
+  const double h = 0.5 * t.dr_je;
+  const cxd w = h * k;
+  const double aw = fabs(w.re) + fabs(w.im);
+  const int nslow = aw <= 1.5 ? max(0, min(np, JE_NEAR - p0)) : np;  // panels 0 .. nslow - 1 of the CTA: sampled
+  int nt = 1;  // terms of the series
+  for (float term = 1.f; nt < JE_NT && term > 1e-19f; ++nt) term *= (float)aw / nt;
+  if (nslow > 0) {
+    for (int x = tid; x < P * P; x += JE_BUILD_THREADS) dct[x] = cospi((double)((x / P) * (x % P)) / (double)M);
+    for (int x = tid; x < nslow * P; x += JE_BUILD_THREADS) {
+      const int lp = x % nslow, n = x / nslow;
+      const cxd lkg = clog_d(0.5 * k) + cxd(0.57721566490153286061, 0.0);
+      // the panel's ends and their sum are exact (make_cheb_je)
+      const double s = (double)(2 * (p0 + lp) + 1) * t.dr_je, u = t.dr_je * cospi((double)n / (double)M);
+      const double r = 0.5 * (s + u);
+      const double dr = 0.5 * (u - (2.0 * r - s));  // |u| <= s: exact
+      cxd j0, j1, g0, g1;
+      je_values(k, lkg, r, dr, j0, j1, g0, g1);
+      if (realk) { j0.im = 0.0; j1.im = 0.0; g0.im = 0.0; g1.im = 0.0; }
+      cxd* o = fv + n * NS * JE_PPC + lp;
+      o[0] = j1;
+      o[JE_PPC] = g1;
+      if (NS == 4) {
+        o[2 * JE_PPC] = j0;
+        o[3 * JE_PPC] = g0;
+      }
+    }
+  }
+  if (warp == 0 && lane >= nslow && lane < np) {
     const cxd lkg = clog_d(0.5 * k) + cxd(0.57721566490153286061, 0.0);
-    const double tn = cospi((double)n / (double)M);
-    const double s = (double)(2 * p + 1) * t.dr_je, u = t.dr_je * tn;
-    const double r = 0.5 * (s + u);
-    const double dr = 0.5 * (u - (2.0 * r - s));  // |u| <= s: exact
-    cxd j0, j1, g0, g1;
-    je_values(k, lkg, r, dr, j0, j1, g0, g1);
-    if (realk) { j0.im = 0.0; j1.im = 0.0; g0.im = 0.0; g1.im = 0.0; }
-    fv[tid][0] = kaL2 * j1;
-    fv[tid][1] = kaL2 * (j1 + cmul_i(g1));
-    if (NS == 4) {
-      fv[tid][2] = kd * j0;
-      fv[tid][3] = kd * (j0 + cmul_i(g0));
+    const double rc = (double)(2 * (p0 + lane) + 1) * h;  // exact
+    cxd a, b, c, d;  // terms n of J0, J1, G0, G1
+    je_values(k, lkg, rc, 0.0, a, b, c, d);
+    if (realk) { a.im = 0.0; b.im = 0.0; c.im = 0.0; d.im = 0.0; }
+    const cxd iz = cinv(rc * k);
+    cxd wa(0.0, 0.0), wc(0.0, 0.0), wd(0.0, 0.0);  // w times terms n - 1
+#pragma unroll 1
+    for (int n = 0; n < nt; ++n) {
+      cxd* o = fv + n * NS * JE_PPC + lane;
+      o[0] = b;
+      o[JE_PPC] = d;
+      if (NS == 4) {
+        o[2 * JE_PPC] = a;
+        o[3 * JE_PPC] = c;
+      }
+      const double n1 = n + 1.0, in = 1.0 / n1, one = n == 0 ? two_over_pi : 0.0;
+      const cxd wn = in * w;
+      const cxd rb = a + iz * (wa - n1 * b);
+      const cxd rc_ = iz * (cxd(one, 0.0) - two_over_pi * a - (double)n * c - wd) - d;
+      const cxd rd = c + iz * (wc - n1 * d - two_over_pi * b);
+      wa = w * a;
+      wc = w * c;
+      wd = w * d;
+      a = -(wn * b);
+      b = wn * rb;
+      c = wn * rc_;
+      d = wn * rd;
     }
   }
   __syncthreads();
-  if (live) {
-    const int m = n, base = lp * P;  // this thread: degree m of panel p
-    const double sg = (m & 1) ? -1.0 : 1.0;
-    double sc = 2.0 / (double)M;
-    if (m == 0) sc *= 0.5;
-    float4* out = t.JE + ((size_t)q * t.nje + p) * (size_t)P * NS;
+  if (lane < np) {
+    const cxd kaL2 = 0.5 * cmul_i(k), kd = -0.5 * k;
+    for (int m = warp; m < P; m += JE_BUILD_THREADS / 32) {
+      cxd acc[NS];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      cxd acc = 0.5 * fv[base][s] + (0.5 * sg) * fv[base + M][s];
-      for (int jn = 1; jn < M; ++jn) acc += dct[jn * P + m] * fv[base + jn][s];
-      acc = sc * acc;
-      const dfl re = df_of(acc.re), im = df_of(acc.im);
-      out[m * NS + s] = make_float4(re.hi, re.lo, im.hi, im.lo);
-      mag[tid][s] = fabs(acc.re) + fabs(acc.im);
+      for (int s = 0; s < NS; ++s) acc[s] = cxd(0.0, 0.0);
+      if (lane < nslow) {
+        const double sg = (m & 1) ? -1.0 : 1.0, sc = (m == 0 || m == M ? 1.0 : 2.0) / (double)M;
+        for (int jn = 0; jn < P; ++jn) {
+          const double cf = sc * (jn == 0 ? 0.5 : jn == M ? 0.5 * sg : dct[jn * P + m]);
+#pragma unroll
+          for (int s = 0; s < NS; ++s) acc[s] += cf * fv[(jn * NS + s) * JE_PPC + lane];
+        }
+      } else {
+        for (int n = m; n < nt; n += 2) {
+          const double cf = g_taylor_to_cheb.c[n][m];
+#pragma unroll
+          for (int s = 0; s < NS; ++s) acc[s] += cf * fv[(n * NS + s) * JE_PPC + lane];
+        }
+      }
+      float4* out = t.JE + (((size_t)q * t.nje + p0 + lane) * P + m) * NS;
+#pragma unroll
+      for (int s = 0; s < NS; s += 2) {
+        const cxd f = s == 0 ? kaL2 : kd;
+        const cxd v[2] = {f * acc[s], f * (acc[s] + cmul_i(acc[s + 1]))};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const dfl re = df_of(v[e].re), im = df_of(v[e].im);
+          out[s + e] = make_float4(re.hi, re.lo, im.hi, im.lo);
+          mag[(m * NS + s + e) * JE_PPC + lane] = fabsf(re.hi) + fabsf(im.hi);
+        }
+      }
     }
   }
   __syncthreads();
-  if (live && n == 0) {
+  if (warp == 0 && lane < np) {
     // FP32 tail: terms from degree m0 on, in every series, sum to at most
     // 2^-26 of the series' coefficient magnitudes; FP32 products of those
     // terms (|T_m| <= 1, error <= 2^-23 each) then stay below 2^-49 of that
     // sum, the order of the double-float rounding of the head (m0 >= 2: the
     // recurrence of the head supplies T_{m0-1} and T_{m0-2})
-    const int base = lp * P;
     int m0 = 2;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      double tot = 0.0;
-      for (int m = 0; m <= M; ++m) tot += mag[base + m][s];
-      double tail = 0.0;
+      auto mg = [&](int m) { return mag[(m * NS + s) * JE_PPC + lane]; };
+      float tot = 0.f, tail = 0.f;
+      for (int m = 0; m <= M; ++m) tot += mg(m);
       int ms = M + 1;
-      while (ms > 2 && tail + mag[base + ms - 1][s] <= 0x1p-26 * tot) tail += mag[base + --ms][s];
+      while (ms > 2 && tail + mg(ms - 1) <= 0x1p-26f * tot) tail += mg(--ms);
       m0 = ms > m0 ? ms : m0;
     }
-    atomicMax(t.JEm + p, m0);
+    atomicMax(t.JEm + p0 + lane, m0);
   }
 }
 
@@ -2184,10 +2271,16 @@ int cheb_je_build(ChebTables& t, const cxd* ks, cudaStream_t st) {
   }
   t.JEm = reinterpret_cast<int*>(t.JE + (size_t)t.nse * t.nk * t.nje * (size_t)(t.Mje + 1));
   QBG_CUDA(cudaMemsetAsync(t.JEm, 0, sizeof(int) * (size_t)t.nje, st));
-  const int ppb = JE_BUILD_THREADS / (t.Mje + 1);
-  dim3 grd((t.nje + ppb - 1) / ppb, t.nk);
-  if (t.nse == 4) k_cheb_build_je<4><<<grd, JE_BUILD_THREADS, 0, st>>>(t, ks);
-  else k_cheb_build_je<2><<<grd, JE_BUILD_THREADS, 0, st>>>(t, ks);
+  const dim3 grd((t.nje + JE_PPC - 1) / JE_PPC, t.nk);
+  auto run = [&](auto ns) -> int {
+    constexpr int NS = decltype(ns)::value;
+    const int smem = (int)je_build_smem<NS>(t.Mje);
+    QBG_CUDA(cudaFuncSetAttribute(k_cheb_build_je<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)je_build_smem<NS>(QBG_CHEB_MAX_DEGREE)));
+    k_cheb_build_je<NS><<<grd, JE_BUILD_THREADS, smem, st>>>(t, ks);
+    return QBG_OK;
+  };
+  QBG_TRY(t.nse == 4 ? run(std::integral_constant<int, 4>{}) : run(std::integral_constant<int, 2>{}));
   QBG_LAUNCH_CHECK("k_cheb_build_je");
   return QBG_OK;
 }
