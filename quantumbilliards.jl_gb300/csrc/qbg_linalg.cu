@@ -2038,9 +2038,14 @@ static LUBatch<T> lu_view(const LUBatch<T>& f, int b0, int cnt) {
 // With extra streams the parts of the batch are factored (solved)
 // concurrently: the panel factorisations and the short GEMM chains of one part
 // leave most SMs idle, which the other parts' kernels fill. The matrices are
-// independent, so the results are those of one stream.
+// independent, so the results are those of one stream. A complex64 batch of
+// less than 2.6e7 elements stays on one stream: its chain of launches is the bound, and
+// every part repeats it (1 / 2 / 4 parts, the whole Beyn call: 16 operators of 256
+// 2.23 / 2.51 / 2.92 ms, 16 of 768 6.21 / 6.60 / 7.19, 24 of 1030 10.2 / 10.4 / 10.9;
+// above it 48 of 768 9.32 / 9.23 / 9.86, 40 of 1030 15.9 / 15.2 / 15.4).
 template <class T>
 static int split_parts(const LUBatch<T>& f) {
+  if (sizeof(T) == 4 && (double)f.batch * f.n * f.n < 2.6e7) return 1;
   return std::max(1, std::min(std::min(f.nsplit, LUBatch<T>::MAX_SPLIT), f.batch));
 }
 
