@@ -986,11 +986,17 @@ __global__ void k_laswp(cx<T>* A, int n, long long stride, int j0, int nb, const
 // lower unit:  inv([A 0; C B]) = [Ai 0; -Bi C Ai  Bi]
 // upper:       inv([A C; 0 B]) = [Ai -Ai C Bi; 0  Bi]
 // A partial last block is padded with the identity.
-// grid (nblocks_to_do, batch); block 256; dynamic smem = 1.25 nb^2 cx<T>
+// grid (nblocks_to_do, batch); block TRTRI_T; dynamic smem = 1.25 nb^2 cx<T>
+// Bound: latency; every panel of a factorisation waits for one. NB = the block size at
+// compile time (0: any), which turns the index divisions into shifts and unrolls the
+// levels. One 64 x 64 complex64 block: 24 us with 256 threads and runtime sizes, 11.5
+// so (16 streamed nodes of N = 5002, 79 panels: 145.3 -> 142.8 ms in all).
 // ---------------------------------------------------------------------------
-template <class T, bool UPPER>
-__global__ void __launch_bounds__(256) k_trtri(const cx<T>* A, int n, long long stride, int nb, int blk0,
-                                               cx<T>* inv, int nblk) {
+constexpr int TRTRI_T = 512;
+template <class T, bool UPPER, int NB>
+__global__ void __launch_bounds__(TRTRI_T) k_trtri(const cx<T>* A, int n, long long stride, int nb_, int blk0,
+                                                   cx<T>* inv, int nblk) {
+  const int nb = NB > 0 ? NB : nb_;
   extern __shared__ unsigned char smraw[];
   cx<T>* S = reinterpret_cast<cx<T>*>(smraw);  // nb x nb, column-major
   cx<T>* Tm = S + nb * nb;                       // scratch, nb*nb/4
@@ -1000,7 +1006,8 @@ __global__ void __launch_bounds__(256) k_trtri(const cx<T>* A, int n, long long 
   const int nr = min(nb, n - r0);
   const cx<T>* a = A + (long long)b * stride;
   const int tid = threadIdx.x;
-  for (int e = tid; e < nb * nb; e += blockDim.x) {
+#pragma unroll 8
+  for (int e = tid; e < nb * nb; e += TRTRI_T) {
     const int i = e % nb, j = e / nb;
     cx<T> v(0, 0);
     if (i < nr && j < nr) {
@@ -1017,11 +1024,12 @@ __global__ void __launch_bounds__(256) k_trtri(const cx<T>* A, int n, long long 
     S[i + j * nb] = v;
   }
   __syncthreads();
-  for (int s = 1; s < nb; s <<= 1) {
+#pragma unroll
+  for (int s = 1; s < (NB > 0 ? NB : nb); s <<= 1) {
     const int npair = nb / (2 * s);
     // T = C * Xi  (lower: C = S[o+s.., o..], Xi = Ai = S[o.., o..])
     //             (upper: C = S[o.., o+s..], Xi = Bi = S[o+s.., o+s..])
-    for (int e = tid; e < npair * s * s; e += blockDim.x) {
+    for (int e = tid; e < npair * s * s; e += TRTRI_T) {
       const int pr = e / (s * s), rem = e % (s * s);
       const int i = rem % s, j = rem / s;
       const int o = pr * 2 * s;
@@ -1034,7 +1042,7 @@ __global__ void __launch_bounds__(256) k_trtri(const cx<T>* A, int n, long long 
       Tm[pr * s * s + i + j * s] = acc;
     }
     __syncthreads();
-    for (int e = tid; e < npair * s * s; e += blockDim.x) {
+    for (int e = tid; e < npair * s * s; e += TRTRI_T) {
       const int pr = e / (s * s), rem = e % (s * s);
       const int i = rem % s, j = rem / s;
       const int o = pr * 2 * s;
@@ -1052,7 +1060,28 @@ __global__ void __launch_bounds__(256) k_trtri(const cx<T>* A, int n, long long 
     __syncthreads();
   }
   cx<T>* out = inv + ((long long)b * nblk + blk) * nb * nb;
-  for (int e = tid; e < nb * nb; e += blockDim.x) out[e] = S[e];
+  for (int e = tid; e < nb * nb; e += TRTRI_T) out[e] = S[e];
+}
+
+template <class T, bool UPPER>
+static int launch_trtri(const cx<T>* A, int n, long long stride, int nb, int blk0, cx<T>* inv, int nblk, int nblocks,
+                        int batch, cudaStream_t st) {
+  const size_t sm = (size_t)nb * nb * sizeof(cx<T>) * 5 / 4;
+  const dim3 grd(nblocks, batch);
+  auto run = [&](auto size) -> int {
+    constexpr int NB = decltype(size)::value;
+    static std::atomic<bool> set{false};
+    if (!set.load()) {
+      QBG_CUDA(cudaFuncSetAttribute(k_trtri<T, UPPER, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+      set.store(true);
+    }
+    k_trtri<T, UPPER, NB><<<grd, TRTRI_T, sm, st>>>(A, n, stride, nb, blk0, inv, nblk);
+    QBG_LAUNCH_CHECK("k_trtri");
+    return QBG_OK;
+  };
+  if (nb == 64) return run(std::integral_constant<int, 64>{});
+  if (nb == 32) return run(std::integral_constant<int, 32>{});
+  return run(std::integral_constant<int, 0>{});
 }
 
 // row permutation from the interchange list (sequential per matrix)
@@ -1455,13 +1484,6 @@ static bool panel_on_cluster(const LUBatch<double>& f, int j0, int w, cudaStream
 template <class T>
 static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first_panel = nullptr) {
   const int n = f.n, nb = f.nb, batch = f.batch;
-  const size_t sm = (size_t)nb * nb * sizeof(cx<T>) * 5 / 4;
-  static bool attr_set[2] = {false, false};
-  if (!attr_set[sizeof(T) == 8]) {
-    QBG_CUDA(cudaFuncSetAttribute(k_trtri<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    QBG_CUDA(cudaFuncSetAttribute(k_trtri<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    attr_set[sizeof(T) == 8] = true;
-  }
   // shared-memory sub-panel width: the widest of 8, 4, 2, 1 columns whose n-row sub-panel fits 160 KiB
   constexpr size_t kPanelSmem = 160 * 1024;
   int sub = 8;
@@ -1500,7 +1522,6 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
     scratch.st = st;
     Lp = scratch.p;
   }
-  const size_t smp = (size_t)pw * pw * sizeof(cx<T>) * 5 / 4;
   auto linv = [&](int j) { return Lp + (long long)(j / pw) * pw * pw; };
   const long long sLinv = (long long)npw * pw * pw;
   for (int J0 = 0; J0 < n; J0 += LU_OUTER * pw) {
@@ -1521,8 +1542,7 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
       dim3 g2((n + 255) / 256, batch);
       k_laswp<T><<<g2, 256, 0, st>>>(f.A, n, f.stride, j0, pw, f.ipiv);
       QBG_LAUNCH_CHECK("k_laswp");
-      k_trtri<T, false><<<dim3(1, batch), 256, smp, st>>>(f.A, n, f.stride, pw, j0 / pw, Lp, npw);
-      QBG_LAUNCH_CHECK("k_trtri lower");
+      QBG_TRY((launch_trtri<T, false>(f.A, n, f.stride, pw, j0 / pw, Lp, npw, 1, batch, st)));
       if (j0 == 0 && after_first_panel) QBG_CUDA(cudaEventRecord(after_first_panel, st));
       const int rin = E - j0 - w;  // columns of this outer block right of the panel
       if (rin > 0) {
@@ -1557,11 +1577,9 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
     }
   }
   if (pw != nb) {
-    k_trtri<T, false><<<dim3(f.nblk, batch), 256, sm, st>>>(f.A, n, f.stride, nb, 0, f.Linv, f.nblk);
-    QBG_LAUNCH_CHECK("k_trtri lower");
+    QBG_TRY((launch_trtri<T, false>(f.A, n, f.stride, nb, 0, f.Linv, f.nblk, f.nblk, batch, st)));
   }
-  k_trtri<T, true><<<dim3(f.nblk, batch), 256, sm, st>>>(f.A, n, f.stride, nb, 0, f.Uinv, f.nblk);
-  QBG_LAUNCH_CHECK("k_trtri upper");
+  QBG_TRY((launch_trtri<T, true>(f.A, n, f.stride, nb, 0, f.Uinv, f.nblk, f.nblk, batch, st)));
   if (sizeof(int) * (size_t)n > 48 * 1024)
     QBG_CUDA(cudaFuncSetAttribute(k_perm_from_ipiv, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(int) * (size_t)n)));
