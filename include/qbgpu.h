@@ -276,11 +276,12 @@ qbg_status qbg_dense_inverse(int32_t n, int32_t batch, int32_t prec, const doubl
                              double* work_out);
 /* Plan of the batched LU, process-wide (no counterpart in the reference):
  * panels per outer block of the two-level factorisation (1..16, default 4;
- * <= 0 keeps the current value), the complex64 panel form (-1 automatic:
- * a cluster of 8 CTAs per panel for batches of at most 4 matrices; 0 one CTA
- * per panel; 1 a cluster) and the number of stream parts a Beyn handle
- * created afterwards factors and solves its operator batch in (1..8,
- * default 4; <= 0 keeps the current value). QBG_LU_OUTER, QBG_LU_CLUSTER and
+ * <= 0 keeps the current value), the panel form (-1 automatic: clusters of
+ * 1 to 16 CTAs, by the rows left for complex64, by rows and batch for
+ * complex128; 0 one CTA per panel; 1 a cluster) and the number of stream
+ * parts a Beyn handle created afterwards factors and solves its operator
+ * batch in (1..8, default 4; <= 0 keeps the current value; complex64 batches
+ * below 2.6e7 elements stay on one stream). QBG_LU_OUTER, QBG_LU_CLUSTER and
  * QBG_LU_SPLIT in the environment give the initial values; qbgpu.autotune
  * chooses them by timing. */
 qbg_status qbg_set_lu_plan(int32_t outer, int32_t cluster, int32_t parts);
@@ -289,10 +290,10 @@ qbg_status qbg_clear_tc_error(void);
 
 /* Smallest singular value of A(k) for nk real wavenumbers (the :svd branch of
  * @svd_or_det_solve, macros.jl:159-161, called by k_sweep,
- * sweepmethods.jl:132-152): FP64 LU of A(k), then block inverse iteration on
- * (A^H A)^{-1} with 8 vectors and a Rayleigh-Ritz step, until the estimate
- * changes by less than 1e-13 relative (at most 40 sweeps); 0 for an exactly
- * singular A(k). */
+ * sweepmethods.jl:132-152): FP64 LU of A(k), then a Lanczos iteration on
+ * (A^H A)^{-1} through the LU factors with full orthogonalisation, until the
+ * Ritz residual is below 1e-12 of the Ritz value (at most 96 steps); 0 for an
+ * exactly singular A(k). */
 qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig);
 
 /* EBIM eigen step at a trial wavenumber k (ebim.jl): the eigenpairs of the

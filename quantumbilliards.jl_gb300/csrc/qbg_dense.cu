@@ -1,8 +1,7 @@
 // FP64 dense building blocks on the library's own kernels: batched LU
-// (k_getrf_panel_smem + k_gemm, qbg_linalg.cu), explicit inverses, and the
-// smallest singular value of A(k) by subspace iteration on A(k)^{-1}, one CTA
-// per matrix with the whole iteration (products, Rayleigh-Ritz, Gram-Schmidt)
-// on the device.
+// (qbg_linalg.cu), explicit inverses, and the smallest singular value of A(k): by
+// subspace iteration on A(k)^{-1} (the inverses' entry and the Newton step), and by
+// a Lanczos iteration on the LU factors (namespace lz below; the sweeps).
 //
 // sigma_min (the reference: svdvals(A)[end], macros.jl:159-161): with
 // C = A^{-1} = V S^{-1} U^H, sigma_min(A) = 1 / sigma_max(C). A block X of

@@ -1,7 +1,7 @@
 // FP64 dense building blocks on the library's own kernels (qbg_dense.cu):
-// batched LU and inverses, the smallest singular value by a device-resident
-// subspace iteration on the inverse, and the deflated shift of the Newton
-// refinement.
+// batched LU and inverses, the smallest singular value by device-resident
+// iterations (on the inverse or on the LU factors), and the deflated shift of the
+// Newton refinement.
 #pragma once
 #include <vector>
 

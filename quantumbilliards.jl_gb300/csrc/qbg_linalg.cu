@@ -5,10 +5,10 @@
 // Algorithm (right-looking blocked LU, the same factorisation LAPACK zgetrf
 // computes; the reference calls lu!(T; check=false), beyn.jl:270-277):
 //   for each block column [j0, j0+nb):
-//     1. k_getf2_panel   one CTA per matrix factors the n-j0 x nb panel
-//                        column by column (pivot = first max of |re|+|im|,
-//                        as izamax); zero pivots are recorded in info and
-//                        skipped, matching check=false.
+//     1. a panel kernel  factors the n-j0 x nb panel column by column on a
+//                        cluster of CTAs or on one (pivot = first max of
+//                        |re|+|im|, as izamax); zero pivots are recorded in
+//                        info and skipped, matching check=false.
 //     2. k_laswp         applies the panel's row interchanges to the columns
 //                        left and right of the panel.
 //     3. k_trtri         inverts the unit-lower diagonal block L11.

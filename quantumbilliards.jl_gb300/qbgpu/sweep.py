@@ -2,7 +2,7 @@
 
 ``k_sweep`` discretises once at max(ks) (sweepmethods.jl:52), builds the
 workspace, and returns sigma_min(A(k)) for every k, computed on the device by
-FP64 LU and block inverse iteration (the reference: LAPACK.gesvd!('N','N',A)[end],
+FP64 LU and a Lanczos iteration on its factors (the reference: LAPACK.gesvd!('N','N',A)[end],
 macros.jl:159-161). ``get_eigenvalues`` is the reference's peak search on the
 second difference of log10(sigma) (sweepmethods.jl:193-217).
 ``newton_refine_svd`` (sweepmethods.jl:307-368) runs on the device
