@@ -495,7 +495,7 @@ def main():
         "roofline": {"bound": "tensor", "achieved": lu_achieved, "peak": bf16, "unit": "TFLOP/s",
                      "frac": lu_achieved / bf16, "traffic": None,
                      "kernel": "LU factor phase of the 48 operators, one disk alone on the device: "
-                               "k_getrf_panel_smem (FP32 panels, CUDA cores) + k_tc_cgemm_pkw trailing updates and "
+                               "k_getrf_panel_f32 (panels, CUDA cores) + k_tc_cgemm_pkw trailing updates and "
                                "k_tc_cgemm in-block products (tcgen05, 3xTF32)",
                      "peak_kind": peak_kind + " bf16 dense (the TF32 tensor rate is half of it and 3xTF32 issues three "
                                               "MMAs per product)",

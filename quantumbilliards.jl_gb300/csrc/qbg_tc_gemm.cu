@@ -44,7 +44,6 @@ constexpr int TC_BN = 32;         // complex columns of C per CTA (real N = 64)
 constexpr int TC_BK = 16;         // complex k per stage (real K = 32 = 4 MMA steps of 8)
 constexpr int TC_KSTEPS = 4;
 constexpr int TC_A_STEP = TC_BM * 8;        // floats per operand block per MMA step (4 KB)
-constexpr int TC_B_STEP = 2 * TC_BN * 8;    // floats (2 KB)
 // the staged kernel's tile widths: 32 complex columns (48 KB stages, two CTAs per
 // SM) or up to 128 (96 KB stages, one)
 template <bool WIDE> struct TS {
