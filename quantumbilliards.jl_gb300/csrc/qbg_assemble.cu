@@ -1755,22 +1755,23 @@ __device__ __noinline__ void je_direct_pair(const GeomDev& g, int i, int j, cxd 
 // low words (the accumulators are unnormalised: hi exact partial sums)
 template <int NS>
 __device__ __forceinline__ void je_series(const float4* __restrict__ c, int M, int m0, dfl t, dfl* v) {
-#pragma unroll
-  for (int s = 0; s < 2 * NS; ++s) v[s] = dfl{0.f, 0.f};
   dfl tp{1.f, 0.f}, tc = t;
   const dfl t2{2.f * t.hi, 2.f * t.lo};
+  // m = 0, 1 (m0 >= 2), with T_0 = 1; inside the loop their tests and the products
+  // with T_0 cost a tenth of it (assembly of 48 nodes of N = 2048 7.1 -> 6.4 ms)
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const float4 c0 = __ldg(c + s), c1 = __ldg(c + NS + s);
+    v[2 * s] = dfl{c0.x, c0.y};
+    v[2 * s + 1] = dfl{c0.z, c0.w};
+    df_acc(v[2 * s], dfl{c1.x, c1.y}, tc);
+    df_acc(v[2 * s + 1], dfl{c1.z, c1.w}, tc);
+  }
 #pragma unroll 2
-  for (int m = 0; m < m0; ++m) {
-    dfl tm;
-    if (m == 0) {
-      tm = tp;
-    } else if (m == 1) {
-      tm = tc;
-    } else {
-      tm = df_sub(df_mul(t2, tc), tp);
-      tp = tc;
-      tc = tm;
-    }
+  for (int m = 2; m < m0; ++m) {
+    const dfl tm = df_sub(df_mul(t2, tc), tp);
+    tp = tc;
+    tc = tm;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       const float4 cc = __ldg(c + m * NS + s);
