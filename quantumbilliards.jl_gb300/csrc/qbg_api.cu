@@ -754,6 +754,7 @@ qbg_status qbg_dense_inverse(int32_t n, int32_t batch, int32_t prec, const doubl
       if (!s) s = lu_factor<double>(D.f, st);
       if (!s) s = D.inverse(Cinv);
       if (!s && sig) s = sigma_iterate(Cinv, n, batch, X0, work, 40, 1e-13, dsig, nullptr, nullptr, st);
+      if (!s) s = tc_check(st);
       if (!s) {
         e = cudaMemcpyAsync(X, Cinv, sizeof(cxd) * nn * batch, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess && sig)

@@ -741,8 +741,7 @@ int Dense64::factor(std::vector<int>* info_host) {
   if (!info_host) return QBG_OK;
   info_host->assign(batch, 0);
   QBG_CUDA(cudaMemcpyAsync(info_host->data(), f.info, sizeof(int) * batch, cudaMemcpyDeviceToHost, st));
-  QBG_CUDA(cudaStreamSynchronize(st));
-  return QBG_OK;
+  return tc_check(st);  // waits for the stream; a product that gave up left its output unwritten
 }
 
 void Dense64::release() {

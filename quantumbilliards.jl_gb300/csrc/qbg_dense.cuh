@@ -31,7 +31,8 @@ struct Dense64 {
   void release();
   cxd* A(int b) const { return f.A + (size_t)b * f.stride; }
   // factors every matrix; info_host (optional) receives LAPACK's info per
-  // matrix (k > 0: U(k, k) == 0), which synchronizes the stream
+  // matrix (k > 0: U(k, k) == 0), which synchronizes the stream and reports
+  // products that gave up on a wait (tc_check)
   int factor(std::vector<int>* info_host = nullptr);
   int inverse(cxd* X) { return lu_inverse<double>(f, X, st); }
   ~Dense64();

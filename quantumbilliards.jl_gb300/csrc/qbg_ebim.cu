@@ -797,7 +797,7 @@ int newton_eval(qbg_geom* g, Newton& W, double k, bool derivs, NewtonEval& out) 
                        derivs ? W.xv : nullptr, E.st));
   if (!derivs) {
     out.lam = sig * sig;
-    return QBG_OK;
+    return tc_check(E.st);
   }
   const cxd one(1, 0), zero(0, 0);
   QBG_TRY(gemm_batched<double>(n, 1, n, one, W.Ac, n, 0, W.xv, n, 0, zero, W.u, n, 0, 1, E.st));     // A x
@@ -842,7 +842,7 @@ int newton_eval(qbg_geom* g, Newton& W, double k, bool derivs, NewtonEval& out) 
   out.lam = lam;
   out.l1 = l1;
   out.l2 = g2 - 2.0 * s2;
-  return QBG_OK;
+  return tc_check(E.st);
 }
 
 qbg_status newton_impl(qbg_geom* g, double k0, double a, double b, int maxiter, double tol, double* k_out,
@@ -1013,7 +1013,7 @@ qbg_status qbg_solve_vect(qbg_geom* g, double k, const double* ds, double* sigma
   QBG_TRY(block_eigs(E, false, p, nev, mu, V, &it, INFINITY));
   std::vector<cxd> hv(n);
   QBG_CUDA(cudaMemcpyAsync(hv.data(), V, sizeof(cxd) * n, cudaMemcpyDeviceToHost, E.st));
-  QBG_TRY(E.wait());
+  QBG_TRY(tc_check(E.st));  // waits for the stream
   double nrm = 0.0;
   for (const cxd& x : hv) nrm += x.re * x.re + x.im * x.im;
   nrm = std::sqrt(nrm);
