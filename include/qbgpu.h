@@ -265,7 +265,8 @@ qbg_status qbg_set_tc_wait_limit(int64_t polls);
 /* Validation entry (no counterpart in the reference): the library's batched
  * LU and explicit inverses of `batch` n x n complex128 matrices (host,
  * column-major, contiguous), X = A^{-1}. prec QBG_PREC_FP64: FP64 LU (the
- * path of sigma_min, EBIM and Newton); with sig != NULL also sigma_min of
+ * path of sigma_min, EBIM and Newton, but with products of fewer than 256 rows
+ * or 64 columns in FP64 throughout: the entries of A may span any range); with sig != NULL also sigma_min of
  * every matrix by the device subspace iteration on its inverse, and with
  * work_out != NULL its final blocks (3 n x 8 complex128 per matrix).
  * prec QBG_PREC_FP32: the matrices rounded to complex64 and factored by the
@@ -312,7 +313,9 @@ qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig)
  * cap). iters (optional, 3 values): iterations of the right and left blocks
  * and the final nev. QBG_ESINGULAR when A(k) is exactly singular.
  * qbg_ebim_eig takes the three N x N complex128 column-major matrices (host,
- * or device with QBG_PTR_DEVICE; left unchanged); qbg_ebim_solve assembles
+ * or device with QBG_PTR_DEVICE; left unchanged), whose entries may span any
+ * range (products below 256 x 64 and the block iteration in FP64 throughout);
+ * qbg_ebim_solve assembles
  * A, A', A'' of the geometry at k on the device first (direct FP64 assembly,
  * as qbg_assemble with deriv = 1). */
 enum { QBG_EBIM_FULL = 8 };

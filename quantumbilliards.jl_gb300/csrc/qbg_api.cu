@@ -748,6 +748,7 @@ qbg_status qbg_dense_inverse(int32_t n, int32_t batch, int32_t prec, const doubl
         !(s = D.alloc(&X0, sizeof(cxd) * (size_t)n * DENSE_P)) && !(s = D.alloc(&dsig, sizeof(double) * batch))) {
       std::vector<cxd> hx;
       dense_start_block(n, hx);
+      D.f.any_range = true;
       cudaError_t e = cudaMemcpyAsync(D.f.A, A, sizeof(cxd) * nn * batch, cudaMemcpyHostToDevice, st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(X0, hx.data(), sizeof(cxd) * hx.size(), cudaMemcpyHostToDevice, st);
       s = e == cudaSuccess ? QBG_OK : cuda_status(e, "qbg_dense_inverse");

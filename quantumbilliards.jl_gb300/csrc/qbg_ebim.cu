@@ -352,6 +352,7 @@ struct Ebim {
   cxd *C = nullptr, *CH = nullptr;  // A^-1 A' and its conjugate transpose
   TcTall tall[2];                   // digit planes of C and CH, made by the first block iteration on them
   Dense64 D;                        // the library's FP64 LU of the matrix in LU
+  bool given = false;               // the matrices are the caller's: no digit products below 256 rows
   std::vector<void*> tmp;
   ~Ebim() {
     if (st) cudaStreamSynchronize(st);
@@ -363,6 +364,7 @@ struct Ebim {
   // LU of the n x n matrix in LU, in place; QBG_ESINGULAR (with what) if U is exactly singular
   int factor(const char* what) {
     QBG_TRY(D.bind(LU, n, 1, st));
+    D.f.any_range = given;
     std::vector<int> info;
     QBG_TRY(D.factor(&info));
     if (info[0] > 0) {
@@ -503,8 +505,9 @@ int block_eigs(Ebim& E, bool adjoint, int p, int nev, std::vector<zc>& mu, cxd* 
   // products on the tensor cores where the FP64 ones take longer than the four
   // launches and the slice sum of a digit product: n^2 p complex FMAs at 2 FP64
   // FMAs per clock and SM reach 50 us at n^2 p = 8e6 (n = 2048, p = 22: 1.40 ms
-  // in FP64, 0.08 ms here; the digits of the operator take 0.2 ms once)
-  const bool tc = (double)n * n * p >= 8e6;
+  // in FP64, 0.08 ms here; the digits of the operator take 0.2 ms once). A caller's
+  // matrices stay in FP64 (see f64_tc in qbg_linalg.cu).
+  const bool tc = !E.given && f64_tc_enabled() && (double)n * n * p >= 8e6;
   TcTall& tall = E.tall[adjoint ? 1 : 0];
   void* xmem = nullptr;
   if (tc) {
@@ -721,6 +724,7 @@ qbg_status qbg_ebim_eig(int64_t n, const void* A, const void* dA, const void* dd
   }
   Ebim E;
   QBG_TRY(ebim_setup(E, (int)n));
+  E.given = true;
   const size_t bytes = sizeof(cxd) * (size_t)n * n;
   QBG_TRY(E.alloc(&E.LU, bytes));
   QBG_TRY(E.alloc(&E.dA, bytes));

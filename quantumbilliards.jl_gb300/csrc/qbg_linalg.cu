@@ -1344,8 +1344,8 @@ void get_lu_plan(int* outer, int* cluster, int* parts) {
 }
 
 // complex128 blocked updates C -= A B on the tensor cores (eight-digit
-// products, tc_gemm_sub_f64) where the product fills the device; QBG_F64_TC=0
-// keeps every FP64 product on the FP64 CUDA-core kernels
+// products, tc_gemm_sub_f64; f64_tc says which); QBG_F64_TC=0 keeps every FP64
+// product on the FP64 CUDA-core kernels
 static std::atomic<int> g_f64_tc{[] {
   const char* e = std::getenv("QBG_F64_TC");
   return (e && *e) ? (std::atoi(e) != 0 ? 1 : 0) : 1;
@@ -1356,15 +1356,24 @@ static std::atomic<int> g_f64_tc{[] {
 // 25 us: from K = 16 on the tensor cores are the faster side down to the
 // smallest products. (24 operators of n = 1502: 32-row products left on the FP64
 // pipe took 53 of 134 ms.)
-static bool f64_tc(int M, int N, int K, int batch) {
-  return g_f64_tc.load() && M >= 16 && N >= 16 && K >= 16 && batch <= 65535;
+//
+// The digits are taken against one maximum per row of A and one per column of B,
+// so a term far below both costs an entry the bits it would keep in FP64: (1, 1e-20)
+// times (1e-20, 1) gives 0. The boundary operators have no such rows (the error of the
+// Beyn, sweep and EBIM results is that of FP64 products); a caller's matrices may
+// (any_range: their rows scaled over 24 decades, n = 200, lost every digit of the inverse),
+// and take digits only where the FP64 kernels cost milliseconds, 256 x 64 and more.
+static bool f64_tc(int M, int N, int K, int batch, bool any_range) {
+  const int m0 = any_range ? 256 : 16, n0 = any_range ? 64 : 16;
+  return g_f64_tc.load() && M >= m0 && N >= n0 && K >= 16 && batch <= 65535;
 }
+bool f64_tc_enabled() { return g_f64_tc.load() != 0; }
 
 template <class T>
 static int gemm_sub(int M, int N, int K, const cx<T>* A, long long lda, long long sA, const cx<T>* B, long long ldb,
-                    long long sB, cx<T>* C, long long ldc, long long sC, int batch, cudaStream_t st) {
+                    long long sB, cx<T>* C, long long ldc, long long sC, int batch, bool any_range, cudaStream_t st) {
   if constexpr (sizeof(T) == 8) {
-    if (f64_tc(M, N, K, batch))
+    if (f64_tc(M, N, K, batch, any_range))
       return tc_gemm_sub_f64(M, N, K, reinterpret_cast<const cxd*>(A), lda, sA, reinterpret_cast<const cxd*>(B), ldb,
                              sB, reinterpret_cast<cxd*>(C), ldc, sC, batch, st);
   }
@@ -1415,9 +1424,9 @@ static int solve_block_mul(int w, int N, const cx<T>* A, int nb, long long sA, c
 // X = A X in place for w x w blocks A: the U rows of the factorisation
 template <class T>
 static int block_mul(int w, int N, const cx<T>* A, long long lda, long long sA, cx<T>* X, long long ldx, long long sX,
-                     int batch, cudaStream_t st) {
+                     int batch, bool any_range, cudaStream_t st) {
   if constexpr (sizeof(T) == 8) {
-    if (f64_tc(w, N, w, batch))
+    if (f64_tc(w, N, w, batch, any_range))
       return tc_block_mul_f64(w, N, reinterpret_cast<const cxd*>(A), lda, sA, reinterpret_cast<cxd*>(X), ldx, sX, batch,
                               st);
   }
@@ -1608,11 +1617,11 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
       const int rin = E - j0 - w;  // columns of this outer block right of the panel
       if (rin > 0) {
         // U12 = inv(L11) A12 and A22 -= L21 U12 on the outer block's columns
-        int s = block_mul<T>(w, rin, linv(j0), pw, sLinv, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, st);
+        int s = block_mul<T>(w, rin, linv(j0), pw, sLinv, f.A + j0 + (long long)(j0 + w) * n, n, f.stride, batch, f.any_range, st);
         if (s) return s;
         s = gemm_sub<T>(n - j0 - w, rin, w, f.A + (j0 + w) + (long long)j0 * n, n, f.stride,
                         f.A + j0 + (long long)(j0 + w) * n, n, f.stride, f.A + (j0 + w) + (long long)(j0 + w) * n, n,
-                        f.stride, batch, st);
+                        f.stride, batch, f.any_range, st);
         if (s) return s;
       }
     }
@@ -1621,19 +1630,19 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
       // U rows of the outer block on the trailing columns: U_b = inv(L_bb) (A_b - sum_{b'<b} L_bb' U_b')
       for (int j0 = J0; j0 < E; j0 += pw) {
         const int w = min(pw, E - j0);
-        int s = block_mul<T>(w, rest, linv(j0), pw, sLinv, f.A + j0 + (long long)E * n, n, f.stride, batch, st);
+        int s = block_mul<T>(w, rest, linv(j0), pw, sLinv, f.A + j0 + (long long)E * n, n, f.stride, batch, f.any_range, st);
         if (s) return s;
         const int below = E - j0 - w;
         if (below > 0) {
           s = gemm_sub<T>(below, rest, w, f.A + (j0 + w) + (long long)j0 * n, n, f.stride,
                           f.A + j0 + (long long)E * n, n, f.stride, f.A + (j0 + w) + (long long)E * n, n, f.stride,
-                          batch, st);
+                          batch, f.any_range, st);
           if (s) return s;
         }
       }
       // trailing update, K = E - J0
       int s = gemm_sub<T>(rest, rest, E - J0, f.A + E + (long long)J0 * n, n, f.stride, f.A + J0 + (long long)E * n,
-                          n, f.stride, f.A + E + (long long)E * n, n, f.stride, batch, st);
+                          n, f.stride, f.A + E + (long long)E * n, n, f.stride, batch, f.any_range, st);
       if (s) return s;
     }
   }
@@ -1755,7 +1764,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
                                 Yc + r0, n, sY, batch, st);
         if (!s && rest > 0)
           s = gemm_sub<T>(rest, Lc, w, f.A + (r0 + w) + (long long)r0 * n, n, f.stride, Yc + r0, n, sY,
-                          Xc + r0 + w, n, sX, batch, st);
+                          Xc + r0 + w, n, sX, batch, f.any_range, st);
         if (s) return s;
       }
       for (int blk = f.nblks - 1; blk >= 0; --blk) {
@@ -1763,7 +1772,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
         int s = gemm_batched<T>(w, Lc, w, one, f.Uinv2 + (long long)blk * bs * bs, bs, sI2, Yc + r0, n, sY, zero,
                                 Xc + r0, n, sX, batch, st);
         if (!s && r0 > 0)
-          s = gemm_sub<T>(r0, Lc, w, f.A + (long long)r0 * n, n, f.stride, Xc + r0, n, sX, Yc, n, sY, batch, st);
+          s = gemm_sub<T>(r0, Lc, w, f.A + (long long)r0 * n, n, f.stride, Xc + r0, n, sX, Yc, n, sY, batch, f.any_range, st);
         if (s) return s;
       }
     }
@@ -1777,7 +1786,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
     const int rest = n - r0 - w;
     if (rest > 0) {
       s = gemm_sub<T>(rest, L, w, f.A + (r0 + w) + (long long)r0 * n, n, f.stride, X + r0, n, sX, X + r0 + w, n, sX,
-                      batch, st);
+                      batch, f.any_range, st);
       if (s) return s;
     }
   }
@@ -1786,7 +1795,7 @@ static int lu_trsolve(const LUBatch<T>& f, int L, cx<T>* X, cudaStream_t st) {
     int s = solve_block_mul<T>(w, L, f.Uinv + (long long)blk * nb * nb, nb, sInv, X + r0, n, sX, batch, st);
     if (s) return s;
     if (r0 > 0) {
-      s = gemm_sub<T>(r0, L, w, f.A + (long long)r0 * n, n, f.stride, X + r0, n, sX, X, n, sX, batch, st);
+      s = gemm_sub<T>(r0, L, w, f.A + (long long)r0 * n, n, f.stride, X + r0, n, sX, X, n, sX, batch, f.any_range, st);
       if (s) return s;
     }
   }

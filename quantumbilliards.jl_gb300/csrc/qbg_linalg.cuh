@@ -15,6 +15,9 @@ struct LUBatch {
   int* ipiv = nullptr;      // batch * n (0-based global row indices, LAPACK order)
   int* perm = nullptr;      // batch * n row permutation (P V gather)
   int* info = nullptr;      // batch
+  // complex128: the entries may span any range (a caller's matrices; see f64_tc in
+  // qbg_linalg.cu). Clear for the boundary operators the library assembles.
+  bool any_range = false;
   cx<T>* Linv = nullptr;    // batch * nblk * nb * nb
   cx<T>* Uinv = nullptr;    // batch * nblk * nb * nb
   // Triangular solves in blocks of nbs = nb * 2^levels rows (levels 0..2):
@@ -162,6 +165,8 @@ int tc_tall_prepare(TcTall& t, const cxd* A, int n, void* mem, cudaStream_t st);
 size_t tc_tall_X_bytes(const TcTall& t, int q);
 int tc_tall_slices(const TcTall& t);
 int tc_tall_product(const TcTall& t, const cxd* X, int q, void* xmem, cxd* P, cudaStream_t st);
+// whether QBG_F64_TC allows complex128 products from digits
+bool f64_tc_enabled();
 // device address of the tensor-core error flag (shared by the GEMM and the residual)
 int tc_error_ptr(int** p);
 
