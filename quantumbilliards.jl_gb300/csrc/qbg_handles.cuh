@@ -8,16 +8,17 @@
 #include "qbg_assemble.cuh"
 
 namespace qbg {
-// caching allocator (qbg_pool.cu)
-int pool_alloc(void** p, size_t bytes);
+// caching allocator (qbg_pool.cu); st: the only stream that will use the block
+// before it is freed there (nullptr: any)
+int pool_alloc(void** p, size_t bytes, cudaStream_t st = nullptr);
 // st: the stream whose work last used p (its completion gates reuse);
 // nullptr waits for the whole device before the block is cached
 void pool_free(void* p, cudaStream_t st);
 
 template <class P>
-inline int dmalloc(P** p, size_t bytes) {
+inline int dmalloc(P** p, size_t bytes, cudaStream_t st = nullptr) {
   void* q = nullptr;
-  const int s = pool_alloc(&q, bytes);
+  const int s = pool_alloc(&q, bytes, st);
   *p = static_cast<P*>(q);
   return s;
 }

@@ -179,7 +179,7 @@ static bool gemm_split_k(int M, int N, int K, cx<T> alpha, const cx<T>* A, long 
   const int kc = ((K + splits - 1) / splits + 15) / 16 * 16;
   const int ns = (K + kc - 1) / kc;
   cx<T>* P = nullptr;
-  if ((*status = dmalloc(&P, sizeof(cx<T>) * (size_t)ns * batch * M * N))) return true;
+  if ((*status = dmalloc(&P, sizeof(cx<T>) * (size_t)ns * batch * M * N, st))) return true;
   {
     dim3 grd((M + 63) / 64, (N + 63) / 64, batch * ns);
     k_gemm_sk<T, CA><<<grd, 256, 0, st>>>(M, N, K, kc, ns, A, lda, sA, B, ldb, sB, P, batch);
@@ -1587,7 +1587,7 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
     ~Scratch() { if (p) dfree(p, st); }
   } scratch;
   if (pw != nb) {
-    QBG_TRY(dmalloc(&scratch.p, sizeof(cx<T>) * (size_t)npw * pw * pw * batch));
+    QBG_TRY(dmalloc(&scratch.p, sizeof(cx<T>) * (size_t)npw * pw * pw * batch, st));
     scratch.st = st;
     Lp = scratch.p;
   }

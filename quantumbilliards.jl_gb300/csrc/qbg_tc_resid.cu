@@ -968,7 +968,7 @@ static int tc_gemm_f64(int M, int N, int K, const cxd* A, long long lda, long lo
     attr[dev] = true;
   }
   unsigned char* mem = nullptr;
-  QBG_TRY(dmalloc(&mem, bytes));
+  QBG_TRY(dmalloc(&mem, bytes, st));
   unsigned char* TDm = mem;
   unsigned char* XDm = mem + td_r;
   int* erow = reinterpret_cast<int*>(mem + td_r + xd_r);
