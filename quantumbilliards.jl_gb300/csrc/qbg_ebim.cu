@@ -93,6 +93,22 @@ __global__ void k_conj_transpose(const cxd* __restrict__ A, cxd* __restrict__ AH
   }
 }
 
+// A <- A^H in place: a CTA exchanges the 32 x 32 tiles (bx, by) and (by, bx), bx <= by
+__global__ void k_conj_transpose_inplace(cxd* A, int n) {
+  __shared__ cxd t[2][32][33];
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32, x = threadIdx.x;
+  if (r0 > c0) return;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    if (r0 + x < n && c0 + j < n) t[0][j][x] = A[(r0 + x) + (size_t)(c0 + j) * n];
+    if (c0 + x < n && r0 + j < n) t[1][j][x] = A[(c0 + x) + (size_t)(r0 + j) * n];
+  }
+  __syncthreads();
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    if (c0 + x < n && r0 + j < n) A[(c0 + x) + (size_t)(r0 + j) * n] = conj(t[0][x][j]);
+    if (r0 + x < n && c0 + j < n) A[(r0 + x) + (size_t)(c0 + j) * n] = conj(t[1][x][j]);
+  }
+}
+
 // Adjoint Fredholm matrix from the Fredholm matrix F = I - D of the DLP:
 // Aadj[a, b] = delta_ab - D[b, a] ds_b / ds_a = F[b, a] ds_b / ds_a (the
 // diagonal ratio is 1). ds: arc-length weights of the full boundary; with a
@@ -349,10 +365,18 @@ struct Ebim {
   cudaStream_t st = nullptr;
   cudaEvent_t ev = nullptr;
   cxd *LU = nullptr, *dA = nullptr, *ddA = nullptr;
-  cxd *C = nullptr, *CH = nullptr;  // A^-1 A' and its conjugate transpose
-  TcTall tall[2];                   // digit planes of C and CH, made by the first block iteration on them
-  Dense64 D;                        // the library's FP64 LU of the matrix in LU
-  bool given = false;               // the matrices are the caller's: no digit products below 256 rows
+  cxd* C = nullptr;      // A^-1 A', or its conjugate transpose
+  bool adjoint = false;  // which of the two
+  // Digit planes of C, 32 n^2 bytes, made again when C changes. They take LU's place where
+  // the factors are no longer needed (lu_free, with room in LU for them), so that
+  // the default form holds 80 n^2 bytes as without planes (144 with those of both
+  // C and C^H beside the five matrices), the full form 96.
+  TcTall tall;
+  void* planes = nullptr;
+  size_t lu_bytes = 0;
+  bool lu_free = false;
+  Dense64 D;           // the library's FP64 LU of the matrix in LU
+  bool given = false;  // the matrices are the caller's: no digit products below 256 rows
   std::vector<void*> tmp;
   ~Ebim() {
     if (st) cudaStreamSynchronize(st);
@@ -378,6 +402,18 @@ struct Ebim {
     int s = dmalloc(q, bytes);
     if (!s) tmp.push_back(*q);
     return s;
+  }
+  // products on the tensor cores where the FP64 ones take longer than the four
+  // launches and the slice sum of a digit product: n^2 p complex FMAs at 2 FP64
+  // FMAs per clock and SM reach 50 us at n^2 p = 8e6 (n = 2048, p = 22: 1.40 ms
+  // in FP64, 0.08 ms here; the digits of the operator take 0.2 ms once). A caller's
+  // matrices stay in FP64 (see f64_tc in qbg_linalg.cu).
+  bool digits(int p) const { return !given && f64_tc_enabled() && (double)n * n * p >= 8e6; }
+  // LU, with room for the planes where a block of p columns takes them and the factors go
+  int alloc_lu(bool goes, int p) {
+    lu_bytes = sizeof(cxd) * (size_t)n * n;
+    if (goes && digits(p)) lu_bytes = std::max(lu_bytes, tc_tall_bytes(n));
+    return alloc(&LU, lu_bytes);
   }
   int wait() {
     cudaError_t e = cudaEventRecord(ev, st);
@@ -502,20 +538,21 @@ int block_eigs(Ebim& E, bool adjoint, int p, int nev, std::vector<zc>& mu, cxd* 
   QBG_TRY(E.alloc(&Y, sizeof(cxd) * np));
   QBG_TRY(E.alloc(&H, sizeof(cxd) * pp));
   QBG_TRY(E.alloc(&Xs, sizeof(cxd) * (size_t)p * nev));
-  // products on the tensor cores where the FP64 ones take longer than the four
-  // launches and the slice sum of a digit product: n^2 p complex FMAs at 2 FP64
-  // FMAs per clock and SM reach 50 us at n^2 p = 8e6 (n = 2048, p = 22: 1.40 ms
-  // in FP64, 0.08 ms here; the digits of the operator take 0.2 ms once). A caller's
-  // matrices stay in FP64 (see f64_tc in qbg_linalg.cu).
-  const bool tc = !E.given && f64_tc_enabled() && (double)n * n * p >= 8e6;
-  TcTall& tall = E.tall[adjoint ? 1 : 0];
+  const bool tc = E.digits(p);
+  TcTall& tall = E.tall;
   void* xmem = nullptr;
+  if (adjoint != E.adjoint) {
+    k_conj_transpose_inplace<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, E.st>>>(E.C, n);
+    QBG_LAUNCH_CHECK("k_conj_transpose_inplace");
+    E.adjoint = adjoint;
+    tall = TcTall();
+  }
   if (tc) {
-    if (!tall.TD) {
-      void* mem = nullptr;
-      QBG_TRY(E.alloc(&mem, tc_tall_bytes(n)));
-      QBG_TRY(tc_tall_prepare(tall, adjoint ? E.CH : E.C, n, mem, E.st));
+    if (!E.planes) {
+      if (E.lu_free && E.lu_bytes >= tc_tall_bytes(n)) E.planes = E.LU;
+      else QBG_TRY(E.alloc(&E.planes, tc_tall_bytes(n)));
     }
+    if (!tall.TD) QBG_TRY(tc_tall_prepare(tall, E.C, n, E.planes, E.st));
     QBG_TRY(E.alloc(&xmem, tc_tall_X_bytes(tall, p)));
     QBG_TRY(E.alloc(&P, sizeof(cxd) * np * tc_tall_slices(tall)));
   } else {
@@ -548,7 +585,7 @@ int block_eigs(Ebim& E, bool adjoint, int p, int nev, std::vector<zc>& mu, cxd* 
       k_sum_slices<<<(unsigned)std::min<size_t>((np + 255) / 256, 4096), 256, 0, E.st>>>(P, tc_tall_slices(tall), np, Y);
       QBG_LAUNCH_CHECK("k_sum_slices");
     } else {
-      QBG_TRY(gemm_nq(adjoint ? E.CH : E.C, Q, Y, n, p, P, E.st));
+      QBG_TRY(gemm_nq(E.C, Q, Y, n, p, P, E.st));
     }
     // Rayleigh-Ritz on the projection Q^H Y
     k_inner<<<p * p, 256, 0, E.st>>>(Q, Y, n, p, H);
@@ -593,13 +630,11 @@ int ebim_run(Ebim& E, double k, double dk, int nev_req, int flags, int cap, doub
   const bool full = (flags & QBG_EBIM_FULL) != 0;
   // LU of A (the reference's lu!(A)), the library's batched FP64 LU with one matrix
   QBG_TRY(E.factor("EBIM: A(k)"));
-  // C = A^-1 A' and C^H from the factors (one solve with n right-hand sides):
-  // every application of the shift-invert operator is then one skinny product
+  // C = A^-1 A' from the factors (one solve with n right-hand sides): every
+  // application of the shift-invert operator is then one skinny product
   QBG_TRY(E.alloc(&E.C, sizeof(cxd) * (size_t)n * n));
-  QBG_TRY(E.alloc(&E.CH, sizeof(cxd) * (size_t)n * n));
   QBG_TRY(lu_solve_shared<double>(E.D.f, E.dA, n, E.C, 0, E.st));
-  k_conj_transpose<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, E.st>>>(E.C, E.CH, n);
-  QBG_LAUNCH_CHECK("k_conj_transpose");
+  E.lu_free = !full;  // the left eigenvectors of the full form take one more solve
   int nev = std::min(nev_req, n);
   std::vector<zc> mur, mul;
   cxd *V = nullptr, *U = nullptr, *W1 = nullptr, *W2 = nullptr;
@@ -932,6 +967,8 @@ int adjoint_into(qbg_geom* g, Ebim& E, double k, const double* ds_host) {
   return E.wait();  // k, the pointer table and ds are staged from this frame
 }
 
+constexpr int VECT_P = 12;  // columns of solve_vect's block iteration
+
 int adjoint_setup(qbg_geom* g, Ebim& E) {
   if (g->d.form != 0 || g->d.quad != 0) {
     set_error("the adjoint Fredholm matrix is defined for the DLP Kress formulation");
@@ -944,9 +981,8 @@ int adjoint_setup(qbg_geom* g, Ebim& E) {
   if (e == cudaSuccess) e = cudaStreamWaitEvent(E.st, ev_in, 0);
   cudaEventDestroy(ev_in);
   if (e != cudaSuccess) return cuda_status(e, "adjoint stream order");
-  const size_t bytes = sizeof(cxd) * (size_t)E.n * E.n;
-  QBG_TRY(E.alloc(&E.LU, bytes));
-  QBG_TRY(E.alloc(&E.C, bytes));
+  QBG_TRY(E.alloc_lu(true, std::min(E.n, VECT_P)));
+  QBG_TRY(E.alloc(&E.C, sizeof(cxd) * (size_t)E.n * E.n));
   return QBG_OK;
 }
 
@@ -1008,8 +1044,9 @@ qbg_status qbg_solve_vect(qbg_geom* g, double k, const double* ds, double* sigma
   QBG_CUDA(cudaMemcpyAsync(E.LU, E.C, sizeof(cxd) * (size_t)n * n, cudaMemcpyDeviceToDevice, E.st));
   QBG_TRY(E.factor("solve_vect: the adjoint Fredholm matrix"));
   QBG_TRY(E.D.inverse(E.C));
+  E.lu_free = true;
   // the eigenvalue of largest modulus of A^-1 (smallest_nullvec_krylov!, dlp.jl:991-1004)
-  const int nev = 1, p = std::min(n, 12);
+  const int nev = 1, p = std::min(n, VECT_P);
   std::vector<zc> mu;
   cxd* V = nullptr;
   int it = 0;
@@ -1047,7 +1084,7 @@ qbg_status qbg_ebim_solve(qbg_geom* g, double k, double dk, int32_t nev, int32_t
   cudaEventDestroy(ev_in);
   if (e != cudaSuccess) return cuda_status(e, "EBIM stream order");
   const size_t bytes = sizeof(cxd) * (size_t)n * n;
-  QBG_TRY(E.alloc(&E.LU, bytes));
+  QBG_TRY(E.alloc_lu(!(flags & QBG_EBIM_FULL), std::min(n, 2 * std::min<int>(nev, n) + 12)));
   QBG_TRY(E.alloc(&E.dA, bytes));
   QBG_TRY(E.alloc(&E.ddA, bytes));
   cxd* dks = nullptr;
