@@ -280,9 +280,9 @@ qbg_status qbg_dense_inverse(int32_t n, int32_t batch, int32_t prec, const doubl
  * <= 0 keeps the current value), the panel form (-1 automatic: clusters of
  * 1 to 16 CTAs, by the rows left for complex64, by rows and batch for
  * complex128; 0 one CTA per panel; 1 a cluster) and the number of stream
- * parts a Beyn handle created afterwards factors and solves its operator
- * batch in (1..8, default 4; <= 0 keeps the current value; complex64 batches
- * below 2.6e7 elements stay on one stream). QBG_LU_OUTER, QBG_LU_CLUSTER and
+ * parts a Beyn handle created afterwards factors and solves its complex64
+ * operator batch in (1..8; 0 keeps the current value; -1, the default: 4, but 1
+ * for a batch below 2.6e7 elements). QBG_LU_OUTER, QBG_LU_CLUSTER and
  * QBG_LU_SPLIT in the environment give the initial values; qbgpu.autotune
  * chooses them by timing. */
 qbg_status qbg_set_lu_plan(int32_t outer, int32_t cluster, int32_t parts);

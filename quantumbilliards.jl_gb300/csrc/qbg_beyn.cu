@@ -50,10 +50,10 @@ struct qbg_beyn {
   std::vector<void*> allocs;
   cudaStream_t st = nullptr;
   // extra streams of the LU and the triangular solves: nsplit parts of the
-  // operator batch run concurrently. QBG_LU_SPLIT in the environment sets the
-  // number of parts (default 4, at most 4; 0 or 1 keeps everything on st);
-  // the results are the same either way
+  // operator batch run concurrently (qbg_set_lu_plan; split_auto: nobody chose the
+  // number); the results are the same either way
   int nsplit = 1;
+  bool split_auto = false;
   cudaStream_t stx[LUBatch<float>::MAX_SPLIT - 1] = {};
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // helper streams of the per-disk QR of the moments (created on first use)
@@ -124,6 +124,7 @@ int setup_lu(qbg_beyn* b, LUBatch<T>& f, int nb, int solve_levels) {
   // the FP64 LU is bound by the FP64 pipe: a second stream only adds contention
   if (sizeof(T) == sizeof(float)) {
     f.nsplit = b->nsplit;
+    f.split_auto = b->split_auto;
     for (int i = 0; i + 1 < b->nsplit; ++i) f.stx[i] = b->stx[i];
     f.ev_fork = b->ev_fork;
     f.ev_join = b->ev_join;
@@ -491,7 +492,8 @@ qbg_status create_impl(qbg_geom* g, const double* k0s, const double* Rs, int ndi
   }
   int parts = 1;
   get_lu_plan(nullptr, nullptr, &parts);  // stream parts of the operator batch (qbg_set_lu_plan)
-  parts = std::max(1, std::min(parts, LUBatch<float>::MAX_SPLIT));
+  b->split_auto = parts < 0;
+  if (parts < 0) parts = 4;
   if (!s && parts > 1) {
     cudaError_t e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);

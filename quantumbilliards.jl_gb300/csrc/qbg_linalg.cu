@@ -1313,7 +1313,8 @@ static int build_solve_blocks(const LUBatch<T>& f, cudaStream_t st) {
 
 // process-wide plan of lu_factor: panels per outer block (1..16), the panel
 // form (-1 automatic, 0 one CTA per panel, 1 a cluster of CTAs) and the
-// number of stream parts a Beyn operator batch is factored and solved in;
+// number of stream parts a Beyn operator batch is factored and solved in (-1
+// automatic, see split_parts);
 // the environment variables QBG_LU_OUTER, QBG_LU_CLUSTER and QBG_LU_SPLIT give
 // the initial values
 static std::atomic<int> g_lu_outer{[] {
@@ -1328,14 +1329,13 @@ static std::atomic<int> g_lu_cluster{[] {
 
 static std::atomic<int> g_lu_parts{[] {
   const char* e = std::getenv("QBG_LU_SPLIT");
-  const int v = (e && *e) ? std::atoi(e) : 4;
-  return std::max(1, std::min(v, LUBatch<float>::MAX_SPLIT));
+  return (e && *e) ? std::max(1, std::min(std::atoi(e), LUBatch<float>::MAX_SPLIT)) : -1;
 }()};
 
 void set_lu_plan(int outer, int cluster, int parts) {
   if (outer > 0) g_lu_outer.store(std::max(1, std::min(outer, 16)));
   g_lu_cluster.store(cluster < 0 ? -1 : (cluster ? 1 : 0));
-  if (parts > 0) g_lu_parts.store(std::min(parts, LUBatch<float>::MAX_SPLIT));
+  if (parts != 0) g_lu_parts.store(parts < 0 ? -1 : std::min(parts, LUBatch<float>::MAX_SPLIT));
 }
 void get_lu_plan(int* outer, int* cluster, int* parts) {
   if (outer) *outer = g_lu_outer.load();
@@ -2126,14 +2126,14 @@ static LUBatch<T> lu_view(const LUBatch<T>& f, int b0, int cnt) {
 // With extra streams the parts of the batch are factored (solved)
 // concurrently: the panel factorisations and the short GEMM chains of one part
 // leave most SMs idle, which the other parts' kernels fill. The matrices are
-// independent, so the results are those of one stream. A complex64 batch of
-// less than 2.6e7 elements stays on one stream: its chain of launches is the bound, and
+// independent, so the results are those of one stream. Automatic: four parts, but
+// one for a complex64 batch of less than 2.6e7 elements, whose chain of launches is the bound:
 // every part repeats it (1 / 2 / 4 parts, the whole Beyn call: 16 operators of 256
 // 2.23 / 2.51 / 2.92 ms, 16 of 768 6.21 / 6.60 / 7.19, 24 of 1030 10.2 / 10.4 / 10.9;
 // above it 48 of 768 9.32 / 9.23 / 9.86, 40 of 1030 15.9 / 15.2 / 15.4).
 template <class T>
 static int split_parts(const LUBatch<T>& f) {
-  if (sizeof(T) == 4 && (double)f.batch * f.n * f.n < 2.6e7) return 1;
+  if (f.split_auto && sizeof(T) == 4 && (double)f.batch * f.n * f.n < 2.6e7) return 1;
   return std::max(1, std::min(std::min(f.nsplit, LUBatch<T>::MAX_SPLIT), f.batch));
 }
 

@@ -37,6 +37,7 @@ struct LUBatch {
   // joined back into the calling stream with these two events
   static constexpr int MAX_SPLIT = 8;
   int nsplit = 1;
+  bool split_auto = false;  // nsplit is a default, which a small batch does not take
   cudaStream_t stx[MAX_SPLIT - 1] = {};
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };

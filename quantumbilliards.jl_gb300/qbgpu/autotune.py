@@ -10,10 +10,11 @@ updates' summation order):
   K = outer * nb), process-wide;
 * ``parts``: contiguous parts of the operator batch factored and solved on
   their own streams, so one part's panels overlap another part's tensor-core
-  updates, process-wide (read when a handle is created);
-* ``cluster``: the panel form: -1 automatic (the 8-CTA cluster panel for
-  batches of at most 4 operators per part, one CTA per panel otherwise),
-  0 always one CTA, 1 the cluster wherever the panel fits it.
+  updates, process-wide (read when a handle is created; complex64 operators
+  only): -1 automatic (four, but one for small batches), or 1 .. 8;
+* ``cluster``: the panel form: -1 automatic (clusters of 1 to 16 CTAs, by the
+  rows left for complex64, by rows and batch for complex128), 0 always one
+  CTA, 1 a cluster wherever the panel fits one (for complex64 the same as -1).
 
 ``tune_beyn`` times whole Beyn steps (assembly, factorisation, solves,
 moments and the host rank test and eigenvalues) of the caller's own workload
@@ -34,7 +35,7 @@ __all__ = ["lu_plan", "set_lu_plan", "tune_beyn"]
 
 
 def lu_plan() -> dict:
-    """The library's current LU plan: outer, cluster (-1 automatic), parts."""
+    """The library's current LU plan: outer, cluster and parts (-1 automatic)."""
     o, c, p = C.c_int32(), C.c_int32(), C.c_int32()
     L.check(L.load().qbg_get_lu_plan(C.byref(o), C.byref(c), C.byref(p)))
     return {"outer": o.value, "cluster": c.value, "parts": p.value}
@@ -83,8 +84,13 @@ def tune_beyn(solver, pts, ws, k0, R, nq, r, mixed=True, cheb=None, svd_tol=1e-1
     cur = lu_plan()
     best = {"nb": nbs[0], "outer": cur["outer"], "parts": cur["parts"], "cluster": -1}
     best["ms"] = run(best["nb"], best["outer"], best["parts"])
-    for p in parts:
-        if p != best["parts"]:
+    # plans that the library runs alike are timed once: the automatic number of
+    # parts, any number of them in FP64, a complex64 panel's cluster
+    single = L.prec_code(mixed) != L.QBG_PREC_FP64
+    auto = 4 if float(nq) * ws.dim ** 2 >= 2.6e7 else 1
+    start = best["parts"] if best["parts"] > 0 else auto
+    for p in parts if single else ():
+        if p != start:
             ms = run(best["nb"], best["outer"], p)
             if ms < best["ms"]:
                 best.update(parts=p, ms=ms)
@@ -101,7 +107,7 @@ def tune_beyn(solver, pts, ws, k0, R, nq, r, mixed=True, cheb=None, svd_tol=1e-1
             if ms < best["ms"]:
                 best.update(nb=nb, outer=o, ms=ms)
     for c in clusters:
-        if c != best["cluster"]:
+        if c != best["cluster"] and not (single and c == 1):
             ms = run(best["nb"], best["outer"], best["parts"], c)
             if ms < best["ms"]:
                 best.update(cluster=c, ms=ms)
