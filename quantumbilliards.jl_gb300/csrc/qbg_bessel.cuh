@@ -31,7 +31,8 @@
 //
 // Accuracy (checked against mpmath in tests/test_gpu_core.py and
 // tests/test_gpu_bessel_panels.py): max error relative to max(|J|,|Y|) below
-// 2e-14, and a few 1e-16 on the Taylor panels.
+// 2e-14, and a few 1e-16 on the Taylor panels; J0 and J1 to 4e-14 of themselves
+// for |z| < 1, Re z > 0 (tests/test_gpu_bessel_small.py).
 //
 // Cost. This part issues 2 FP64 FMAs per clock and SM, so an evaluation costs
 // its FP64 instruction count and nothing else: the recurrence takes about
@@ -344,6 +345,19 @@ constexpr HankelCoef hankel_coef() {
   return h;
 }
 
+// On panel 0 the derivative series leaves J1 an absolute error of a few 1e-16
+// (5e-13 of J1 at 1e-3, 5e-8 at 1e-8); below 0.25 the power series
+// (z/2) sum (-z^2/4)^m / (m! (m+1)!) keeps it to rounding in six terms (q = -z^2/4).
+constexpr double BP_SMALL = 0.25;
+template <class T>
+__device__ __forceinline__ T j1_small(T z, T q) {
+  T s = q * (1.0 / 86400.0) + T(1.0 / 2880.0);
+  s = s * q + T(1.0 / 144.0);
+  s = s * q + T(1.0 / 12.0);
+  s = s * q + T(0.5);
+  return 0.5 * (z * (s * q + T(1.0)));
+}
+
 // J0, J1, Y0, Y1 at a real x > 0
 struct Bessel01r {
   double j0, j1, y0, y1;
@@ -369,6 +383,7 @@ __device__ __forceinline__ Bessel01r bessel01_real(double x) {
     r.j0 = a;
     r.j1 = -ap;
     if (n < BP_G) {
+      if (x < BP_SMALL) r.j1 = j1_small(x, -0.25 * x * x);
       const double l = two_over_pi * log(x);
       r.y0 = fma(l, a, b);
       r.y1 = fma(l, r.j1, -two_over_pi * a / x) - bp;
@@ -442,7 +457,9 @@ static __device__ __noinline__ Bessel01d bessel01_panel(cxd z) {
   r.j0 = j0;
   r.j1 = -jp;
   if (n < BP_G) {
-    const cxd l = two_over_pi * cxd(log(hypot(z.re, z.im)), atan2(z.im, z.re));
+    const double az = hypot(z.re, z.im);
+    if (az < BP_SMALL) r.j1 = j1_small(z, -0.25 * (z * z));
+    const cxd l = two_over_pi * cxd(log(az), atan2(z.im, z.re));
     r.y0 = g0 + l * j0;
     r.y1 = l * r.j1 - two_over_pi * (j0 * cinv(z)) - gp;
   } else {
