@@ -293,8 +293,10 @@ qbg_status qbg_clear_tc_error(void);
  * @svd_or_det_solve, macros.jl:159-161, called by k_sweep,
  * sweepmethods.jl:132-152): FP64 LU of A(k), then a Lanczos iteration on
  * (A^H A)^{-1} through the LU factors with full orthogonalisation, until the
- * Ritz residual is below 1e-12 of the Ritz value (at most 96 steps); 0 for an
- * exactly singular A(k). */
+ * Ritz residual is below 1e-12 of the Ritz value (at most 96 steps, which only an
+ * operator whose smallest singular values crowd together reaches; the value is
+ * then an upper bound); 0 for an exactly singular A(k), NaN for one with entries
+ * that are not finite. */
 qbg_status qbg_sigma_min(qbg_geom* g, const double* ks, int64_t nk, double* sig);
 
 /* EBIM eigen step at a trial wavenumber k (ebim.jl): the eigenpairs of the

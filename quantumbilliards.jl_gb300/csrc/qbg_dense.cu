@@ -618,8 +618,10 @@ __global__ void __launch_bounds__(T, 2) k_lanczos_sigma(const cxd* LU, const cxd
   o.n = n;
   o.nblk = nblk;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (info[mat] > 0) {  // singular (the whole cluster leaves): sigma_min = 0
-    if (o.rank == 0 && tid == 0) sig[mat] = 0.0;
+  if (info[mat] > 0) {  // no pivot (the whole cluster leaves): sigma_min = 0 at an exact zero, else the column is NaN
+    const cxd u = o.A[(size_t)(info[mat] - 1) * (n + 1)];
+    if (o.rank == 0 && tid == 0)
+      sig[mat] = u.re == 0.0 && u.im == 0.0 ? 0.0 : __longlong_as_double(0x7FF8000000000000ll);
     return;
   }
   cxd* V = work + (size_t)mat * per;
@@ -703,7 +705,8 @@ __global__ void __launch_bounds__(T, 2) k_lanczos_sigma(const cxd* LU, const cxd
       if (end || !(beta * sres[1] > tol * theta)) break;
     }
   }
-  if (o.rank == 0 && tid == 0) sig[mat] = theta > 0.0 && isfinite(theta) ? 1.0 / sqrt(theta) : 0.0;
+  // a NaN here (an infinite entry of A) stays one: 0 is the answer of a singular operator
+  if (o.rank == 0 && tid == 0) sig[mat] = 1.0 / sqrt(theta);
 }
 
 }  // namespace lz

@@ -43,7 +43,8 @@ struct Dense64 {
 int sigma_iterate(const cxd* Cinv, int n, int batch, const cxd* X0, cxd* work, int maxit, double tol, double* sig,
                   int* iters, cxd* vec, cudaStream_t st);
 // sigma_min of every A_b of a factored batch (nb = 64, levels = 0) straight from
-// the factors, by Lanczos on (A A^H)^{-1} (see qbg_dense.cu); 0 where info > 0;
+// the factors, by Lanczos on (A A^H)^{-1} (see qbg_dense.cu); 0 where a pivot is 0,
+// NaN where an entry is not finite;
 // tol: the Ritz residual relative to the Ritz value; work: batch * sigma_lu_work(n)
 // elements.
 size_t sigma_lu_work(int n);
