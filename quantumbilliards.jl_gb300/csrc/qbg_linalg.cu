@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 #include <cstdlib>
 #include <type_traits>
+#include "qbg_device_flag.cuh"
 #include "qbg_linalg.cuh"
 #include "qbg_handles.cuh"
 
@@ -1123,6 +1124,17 @@ __global__ void __launch_bounds__(TRTRI_T) k_trtri(const cx<T>* A, int n, long l
   for (int e = tid; e < nb * nb; e += TRTRI_T) out[e] = S[e];
 }
 
+// the kernel's limit of dynamic shared memory, once per device; a refusal is reported by every call
+static int smem_limit(DeviceFlag& set, const void* kernel, int bytes) {
+  int dev = 0;
+  QBG_CUDA(cudaGetDevice(&dev));
+  cudaError_t e = cudaSuccess;
+  auto ask = [&] { return (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) == cudaSuccess; };
+  if (!set.get(dev, ask) && e == cudaSuccess) ask();
+  QBG_CUDA(e);
+  return QBG_OK;
+}
+
 template <class T, bool UPPER>
 static int launch_trtri(const cx<T>* A, int n, long long stride, int nb, int blk0, cx<T>* inv, int nblk, int nblocks,
                         int batch, cudaStream_t st) {
@@ -1130,11 +1142,8 @@ static int launch_trtri(const cx<T>* A, int n, long long stride, int nb, int blk
   const dim3 grd(nblocks, batch);
   auto run = [&](auto size) -> int {
     constexpr int NB = decltype(size)::value;
-    static std::atomic<bool> set{false};
-    if (!set.load()) {
-      QBG_CUDA(cudaFuncSetAttribute(k_trtri<T, UPPER, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-      set.store(true);
-    }
+    static DeviceFlag set;
+    QBG_TRY(smem_limit(set, (const void*)k_trtri<T, UPPER, NB>, 96 * 1024));
     k_trtri<T, UPPER, NB><<<grd, TRTRI_T, sm, st>>>(A, n, stride, nb, blk0, inv, nblk);
     QBG_LAUNCH_CHECK("k_trtri");
     return QBG_OK;
@@ -1435,8 +1444,8 @@ static int block_mul(int w, int N, const cx<T>* A, long long lda, long long sA, 
 
 // Whether clusters of cs CTAs can run the kernel with smem bytes of dynamic
 // shared memory (its attributes are set here; more than 8 CTAs only where the
-// occupancy query finds room)
-static bool cluster_kernel_ok(const void* kernel, int cs, int threads, int smem) {
+// occupancy query finds room); asked once per device
+static bool cluster_kernel_ask(const void* kernel, int cs, int threads, int smem) {
   bool k = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
   if (k && cs > 8) {
     k = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
@@ -1452,12 +1461,17 @@ static bool cluster_kernel_ok(const void* kernel, int cs, int threads, int smem)
   (void)cudaGetLastError();  // a refused attribute or query leaves this size off, nothing else
   return k;
 }
+static bool cluster_kernel_ok(DeviceFlag& flag, const void* kernel, int cs, int threads, int smem) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  return flag.get(dev, [&] { return cluster_kernel_ask(kernel, cs, threads, smem); });
+}
 
 template <int CS>
 static bool panel_cluster_ok() {
-  static const bool ok = cluster_kernel_ok((const void*)k_getrf_panel_cluster<double, CS>, CS, PC_THREADS,
-                                           pc_max_rpc<double, CS>(32) * 32 * (int)sizeof(cxd));
-  return ok;
+  static DeviceFlag flag;
+  return cluster_kernel_ok(flag, (const void*)k_getrf_panel_cluster<double, CS>, CS, PC_THREADS,
+                           pc_max_rpc<double, CS>(32) * 32 * (int)sizeof(cxd));
 }
 
 template <int CS>
@@ -1506,8 +1520,8 @@ static int panel_cluster_size_f64(int n, int batch, int w) {
 
 template <int CS>
 static bool panel_f32_ok() {
-  static const bool ok = cluster_kernel_ok((const void*)k_getrf_panel_f32<CS>, CS, FP_T, FP_ROWS * 64 * (int)sizeof(cxf));
-  return ok;
+  static DeviceFlag flag;
+  return cluster_kernel_ok(flag, (const void*)k_getrf_panel_f32<CS>, CS, FP_T, FP_ROWS * 64 * (int)sizeof(cxf));
 }
 
 // 0: the one-CTA kernel
@@ -1558,12 +1572,8 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   int sub = 8;
   while (sub > 1 && (size_t)n * sub * sizeof(cx<T>) > kPanelSmem) sub >>= 1;
   const bool smem_panel = (size_t)n * sub * sizeof(cx<T>) <= kPanelSmem;
-  static bool panel_attr[2] = {false, false};
-  if (smem_panel && !panel_attr[sizeof(T) == 8]) {
-    QBG_CUDA(cudaFuncSetAttribute(k_getrf_panel_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kPanelSmem));
-    panel_attr[sizeof(T) == 8] = true;
-  }
+  static DeviceFlag panel_attr;
+  if (smem_panel) QBG_TRY(smem_limit(panel_attr, (const void*)k_getrf_panel_smem<T>, (int)kPanelSmem));
   // complex128 panels are 32 columns wide whatever the block size of the
   // inverses: half of a 64-column panel's FP64 work is its second half's
   // update, which the tensor cores do in a fraction of the time
