@@ -279,7 +279,7 @@ int make_cheb(qbg_geom* g, const cxd* dks, int nk, const qbg_cheb_params& prm, C
 // carry up to ~2.4x the interpolation error of J0, J1 on the same panels, and
 // 1.5x more panels lower it by 1.5^(M+1) (11x at M = 5, 58x at M = 9), so the
 // tables are at least as accurate as the reference's J tables
-int make_cheb_je(qbg_geom* g, const cxd* dks, int nk, const qbg_cheb_params& prm, ChebTables& t,
+int make_cheb_je(qbg_geom* g, const cxd* dks, int nk, double kmax, const qbg_cheb_params& prm, ChebTables& t,
                  std::vector<void*>& tmp, cudaStream_t st) {
   double lo = 0, hi = 0;
   QBG_TRY(cheb_range(g, tmp, st, &lo, &hi));
@@ -289,11 +289,19 @@ int make_cheb_je(qbg_geom* g, const cxd* dks, int nk, const qbg_cheb_params& prm
   t.rmin = 0.95 * lo;
   t.rmax = 1.05 * hi;
   t.small_cut = 0.0;
-  // twice for a reduced operator below degree 9, which takes J/E tables only where
-  // the H panels set its error before: 1.5 times left it at 4.4e-14 (rms of the
-  // assembled operator, degree 7, N = 4096, k = 300) against the H and J tables' 1.4e-14
-  const long long f = (g->d.m != g->d.n && prm.M_j < 9) ? 4 : 3;
-  t.nje = (int)std::min<long long>((f * prm.n_panels_j + 1) / 2, (1LL << 21) - 1);
+  long long nje = (3LL * prm.n_panels_j + 1) / 2;
+  if (g->d.m != g->d.n) {
+    // A reduced operator's images take the H panels' error alone on the H and J
+    // tables, so its J/E panels do not follow n_panels_j: they are so narrow that
+    // the terms past degree M, at most 2 (w/2)^(M+1) / (M+1)! with w = |k| times half a
+    // width, are below rounding, but no more than the two tables had together.
+    // rms error of the assembled operator, N = 2048, k = 150, panels (1520, 10, 203, 10):
+    // 5.9e-13 with 1.5 n_panels_j, 3.9e-14 on the H and J tables.
+    const double w = 2.0 * std::pow(0x1p-54 * std::tgamma(prm.M_j + 2.0), 1.0 / (prm.M_j + 1.0));
+    const double need = std::ceil(kmax * t.rmax / (2.0 * w)), most = (double)prm.n_panels_h + prm.n_panels_j;
+    nje = std::max(nje, (long long)std::min(need, most));
+  }
+  t.nje = (int)std::min<long long>(nje, (1LL << 21) - 1);
   t.Mje = prm.M_j;
   // a width of 30 bits (rounded up, 2^-30 at most), so that the ends of every panel
   // and their sums are exact and a radius keeps its place in the panel
@@ -330,6 +338,8 @@ static int assemble_impl(qbg_geom* g, const double* ks, int64_t nk, int32_t deri
     return QBG_EINVAL;
   }
   QBG_TRY(check_ks(ks, nk));
+  double kmax = 0.0;
+  for (int64_t q = 0; q < nk; ++q) kmax = std::max(kmax, std::hypot(ks[2 * q], ks[2 * q + 1]));
   std::lock_guard<std::mutex> lk(g->mu);
   const int64_t dim = g->dim;
   const size_t esz = prec ? sizeof(cxf) : sizeof(cxd);
@@ -368,7 +378,7 @@ static int assemble_impl(qbg_geom* g, const double* ks, int64_t nk, int32_t deri
       std::vector<void*> ctmp;
       ChebTables t;
       if (cheb_je_applies(g->d, deriv, prec, *cheb)) {
-        s = make_cheb_je(g, dks + k0, (int)c, *cheb, t, ctmp, st);
+        s = make_cheb_je(g, dks + k0, (int)c, kmax, *cheb, t, ctmp, st);
       } else {
         s = make_cheb(g, dks + k0, (int)c, *cheb, t, ctmp, st);
         if (!s && prec != QBG_PREC_FP64 && cheb_df_applies(g->d, deriv)) s = make_cheb_df(t, dks + k0, ctmp, st);

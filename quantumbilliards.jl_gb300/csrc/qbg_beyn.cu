@@ -37,6 +37,7 @@ struct qbg_beyn {
   int prec = 0;
   qbg_beyn_opts opts{};
   cxd* zj = nullptr;  // device contour nodes (nn)
+  double kmax = 0.0;  // the largest of their moduli
   cxd* wj = nullptr;  // device contour weights (nn)
   LUBatch<double> fd;  // FP64 form: cap operators
   LUBatch<float> ff;   // complex64 forms: cap operators
@@ -148,6 +149,7 @@ int setup(qbg_beyn* b, const double* k0s, const double* Rs) {
       const double th = 2.0 * M_PI * (double)j / (double)nq;
       const double c = std::cos(th), s = std::sin(th);
       z[d * nq + j] = cxd(k0r + R * c, k0i + R * s);
+      b->kmax = std::max(b->kmax, std::hypot(k0r + R * c, k0i + R * s));
       w[d * nq + j] = cxd((R / nq) * c, (R / nq) * s);
     }
   }
@@ -217,7 +219,7 @@ int load(qbg_beyn* b, int n0, int c) {
     ChebTables t;
     int s = QBG_OK;
     if (cheb_je_applies(b->g->d, 0, b->prec, cp)) {
-      s = make_cheb_je(b->g, b->zj + n0, c, cp, t, ctmp, st);
+      s = make_cheb_je(b->g, b->zj + n0, c, b->kmax, cp, t, ctmp, st);
     } else {
       s = make_cheb(b->g, b->zj + n0, c, cp, t, ctmp, st);
       if (!s && b->prec != QBG_PREC_FP64 && cheb_df_applies(b->g->d, 0)) s = make_cheb_df(t, b->zj + n0, ctmp, st);
