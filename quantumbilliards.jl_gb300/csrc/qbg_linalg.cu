@@ -1576,8 +1576,11 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   if (smem_panel) QBG_TRY(smem_limit(panel_attr, (const void*)k_getrf_panel_smem<T>, (int)kPanelSmem));
   // complex128 panels are 32 columns wide whatever the block size of the
   // inverses: half of a 64-column panel's FP64 work is its second half's
-  // update, which the tensor cores do in a fraction of the time
-  const int pw = sizeof(T) == 8 ? std::min(nb, 32) : nb;
+  // update, which the tensor cores do in a fraction of the time. Not where the
+  // short products stay in FP64 (any_range): those cost as much outside the panel,
+  // in twice the launches (inverse of 2 matrices of 700: 19.7 ms with 32 columns, 15.0
+  // with 64)
+  const int pw = sizeof(T) == 8 && !f.any_range ? std::min(nb, 32) : nb;
   QBG_CUDA(cudaMemsetAsync(f.info, 0, sizeof(int) * batch, st));
   // two-level right-looking LU: panels of nb columns inside outer blocks of
   // LU_OUTER panels. A panel's updates reach only the columns of its outer
