@@ -1050,10 +1050,18 @@ __global__ void __launch_bounds__(256) k_assemble_cfie_reduced(GeomDev g, ChebTa
 
 // reduced CFIE launcher: cheb == nullptr evaluates the kernels directly;
 // prec QBG_PREC_FP32 writes complex64 values without low words
+// CTA of the direct kernels with one entry per thread: 64 threads where 256 would
+// leave SMs without a CTA. FP64 instructions of the warps of one SM quarter run one
+// after another, and at complex k a warp whose entries lie inside and outside the
+// Taylor panels' strip takes both ways (mixed form, k + 0.3i: n = 64
+// 168 -> 106 us, reduced to 16 697 -> 388; n = 192, 144 CTAs of 256, 229 -> 143)
+static dim3 entry_block(int dim) { return dim3(32, (dim + 31) / 32 * ((dim + 7) / 8) < 152 ? 2 : 8); }
+
 static int launch_cfie_reduced(const GeomDev& g, const ChebTables* cheb, const cxd* ks, int nk, int deriv, int prec,
                                void* const* outs_dev, void* const* lo_outs_dev, long long ld, cudaStream_t st) {
   const int kchunk = 8;
-  dim3 blk(32, 8), grd((g.m + 31) / 32, (g.m + 7) / 8, (nk + kchunk - 1) / kchunk);
+  const dim3 blk = cheb ? dim3(32, 8) : entry_block(g.m);
+  const dim3 grd((g.m + blk.x - 1) / blk.x, (g.m + blk.y - 1) / blk.y, (nk + kchunk - 1) / kchunk);
   const ChebTables t0 = cheb ? *cheb : ChebTables();
   void* const* lo = prec == QBG_PREC_MIXED ? lo_outs_dev : nullptr;
 #define QBG_CFR(D, O, C) k_assemble_cfie_reduced<D, O, C><<<grd, blk, 0, st>>>(g, t0, ks, nk, kchunk, outs_dev, lo, ld)
@@ -2596,8 +2604,7 @@ int launch_assemble(const GeomDev& g, const cxd* ks, int nk, int deriv, int prec
                     long long ld, cudaStream_t st, void* const* lo_outs_dev) {
   const bool reduced = (g.m != g.n);
   const int dim = reduced ? g.m : g.n;
-  dim3 blk(32, 8);
-  dim3 grd((dim + 31) / 32, (dim + 7) / 8);
+  const dim3 blk = entry_block(dim), grd((dim + blk.x - 1) / blk.x, (dim + blk.y - 1) / blk.y);
   if (g.quad == 1) return launch_alpert(g, nullptr, ks, nk, deriv, prec, outs_dev, ld, st, lo_outs_dev);
   if (reduced) {
     if (g.form != 0) return launch_cfie_reduced(g, nullptr, ks, nk, deriv, prec, outs_dev, lo_outs_dev, ld, st);
