@@ -277,7 +277,8 @@ qbg_status qbg_dense_inverse(int32_t n, int32_t batch, int32_t prec, const doubl
                              double* work_out);
 /* Plan of the batched LU, process-wide (no counterpart in the reference):
  * panels per outer block of the two-level factorisation (1..16, default 4;
- * <= 0 keeps the current value), the panel form (-1 automatic: clusters of
+ * <= 0 keeps the current value; complex64 panels have the block size's columns,
+ * complex128 panels 32 whatever it is), the panel form (-1 automatic: clusters of
  * 1 to 16 CTAs, by the rows left for complex64, by rows and batch for
  * complex128; 0 one CTA per panel; 1 a cluster) and the number of stream
  * parts a Beyn handle created afterwards factors and solves its complex64
@@ -445,8 +446,8 @@ qbg_status qbg_serve_destroy(qbg_server* s);
  * b < batch, column-major host buffers (complex interleaved floats; A_b at
  * A + 2*b*lda*K, B_b at B + 2*b*ldb*N, C_b at C + 2*b*ldc*N). engine selects
  * the GEMM inside the FP32 LU and solves: 0 = CUDA-core FMA tiles,
- * 1 = tcgen05 tensor cores (3xTF32; for products of at least 4 x 8 output
- * tiles the operands are packed once per call into split tile images that
+ * 1 = tcgen05 tensor cores (3xTF32; for products of at least 10 x 10 output
+ * tiles of 128 x 128, more than 152 over the batch, and K >= 32 the operands are packed once per call into split tile images that
  * bulk copies stream through a four-stage ring, smaller ones split their
  * operands in registers), 2 = tcgen05 with operands split in registers always. No reference counterpart: the reference's
  * GEMMs run inside LAPACK's getrf/getrs (beyn.jl:270-280). */

@@ -1048,15 +1048,15 @@ __global__ void __launch_bounds__(256) k_assemble_cfie_reduced(GeomDev g, ChebTa
   }
 }
 
-// reduced CFIE launcher: cheb == nullptr evaluates the kernels directly;
-// prec QBG_PREC_FP32 writes complex64 values without low words
 // CTA of the direct kernels with one entry per thread: 64 threads where 256 would
 // leave SMs without a CTA. FP64 instructions of the warps of one SM quarter run one
 // after another, and at complex k a warp whose entries lie inside and outside the
 // Taylor panels' strip takes both ways (mixed form, k + 0.3i: n = 64
-// 168 -> 106 us, reduced to 16 697 -> 388; n = 192, 144 CTAs of 256, 229 -> 143)
+// 168 -> 106 us, reduced to 16 697 -> 388)
 static dim3 entry_block(int dim) { return dim3(32, (dim + 31) / 32 * ((dim + 7) / 8) < 152 ? 2 : 8); }
 
+// reduced CFIE launcher: cheb == nullptr evaluates the kernels directly;
+// prec QBG_PREC_FP32 writes complex64 values without low words
 static int launch_cfie_reduced(const GeomDev& g, const ChebTables* cheb, const cxd* ks, int nk, int deriv, int prec,
                                void* const* outs_dev, void* const* lo_outs_dev, long long ld, cudaStream_t st) {
   const int kchunk = 8;

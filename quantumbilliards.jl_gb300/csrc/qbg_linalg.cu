@@ -538,23 +538,26 @@ __global__ void __launch_bounds__(1024) k_getrf_panel_smem(cx<T>* A, int n, long
 }
 
 // ---------------------------------------------------------------------------
-// Panel factorisation on a cluster of PC_CS CTAs per matrix: the m x w panel
+// complex128 panel on a cluster of PC_CS CTAs per matrix (panel_cluster_size_f64
+// says how many): the m x w panel
 // (m = n - j0 rows, w <= 64 columns) is held in the CTAs' shared memory, rows
 // in blocks of rpc = ceil(m / PC_CS) per CTA. One cluster barrier per column:
 // before it, every CTA pushes into every CTA's shared memory its candidate
 // (the largest |re| + |im| of the column over its rows at or below the
 // diagonal, lowest row on ties, as izamax) together with that whole candidate
 // row, and the owner of the diagonal row pushes the diagonal row; after it,
-// every CTA picks the pivot from the eight candidates locally, so the pivot
+// every CTA picks the pivot from the PC_CS candidates locally, so the pivot
 // row and the displaced row are already on chip, the two owners write the
 // interchange into their rows and every CTA scales and updates its own rows.
 // The push buffers alternate between two copies by column parity: a CTA
 // pushing column c + 1 writes the other copy than the one a slower CTA may
 // still read for column c, and cannot reach column c + 2 before that CTA has
 // passed the barrier of column c + 1. Same factors, pivots and info as
-// k_getrf_panel_smem. (Measured on 2048 x 64 panels: 228 us with 256 threads
-// per CTA; 1024 threads sharing each row's columns took 274 us, the per-thread
-// pivot bookkeeping then outweighing the split update.)
+// k_getrf_panel_smem.
+// Bound by latency where few operators leave it 16 CTAs each: about 10 us a
+// column of a 2048 x 32 panel, four to five block barriers, the cluster barrier
+// and the update through shared memory; by FP64 issue where the batch fills the
+// SMs with one or two CTAs each.
 // ---------------------------------------------------------------------------
 constexpr int PC_THREADS = 256;
 // largest rows per CTA of a panel of w columns: what the push buffers, whose
@@ -714,7 +717,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(PC_THREADS)
 // The factors, pivots (first index on ties) and info are those of
 // column-by-column partial pivoting.
 //
-// Bound by latency: one block and one cluster barrier per column, about 1.6 us.
+// Bound by latency: one block and one cluster barrier per column, 2.3 to 2.5 us.
 // Measured per 64-column panel: 145-160 us at up to 3200 rows, 190 us at 5000
 // (16 CTAs); the one-CTA kernel takes 340-460 us at 2048 rows, the cluster form
 // that keeps the panel in shared memory column by column 190-340 us.
@@ -1582,11 +1585,12 @@ static int lu_factor_one(LUBatch<T>& f, cudaStream_t st, cudaEvent_t after_first
   // with 64)
   const int pw = sizeof(T) == 8 && !f.any_range ? std::min(nb, 32) : nb;
   QBG_CUDA(cudaMemsetAsync(f.info, 0, sizeof(int) * batch, st));
-  // two-level right-looking LU: panels of nb columns inside outer blocks of
+  // two-level right-looking LU: panels of pw columns inside outer blocks of
   // LU_OUTER panels. A panel's updates reach only the columns of its outer
   // block; the trailing matrix right of an outer block is updated once, with
-  // K = LU_OUTER * nb, after the outer block's U rows are formed by block
-  // forward substitution (the nb x nb inverses of L from k_trtri). The row
+  // K = LU_OUTER * pw, after the outer block's U rows are formed by block
+  // forward substitution (the pw x pw inverses of L from k_trtri; where pw < nb
+  // the nb x nb inverses that the solves take are made at the end). The row
   // interchanges of every panel still apply to all columns at once (k_laswp),
   // so the factors are those of the one-level algorithm.
   // panels per outer block: set_lu_plan (or QBG_LU_OUTER in the environment), 1..16, default 4

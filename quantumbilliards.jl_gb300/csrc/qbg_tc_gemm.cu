@@ -660,8 +660,8 @@ int* g_tc_err_addr[TC_MAX_DEV] = {};
 bool g_tc_attr[TC_MAX_DEV] = {};
 std::atomic<int> g_engine{GEMM_ENGINE_TCGEN05};
 std::atomic<bool> g_pk_enabled{true};  // packed-operand path of tc_gemm_c64
-// wide-tile packed path: QBG_GEMM_WIDE in the environment, 0 keeps the
-// 128 x 32 tiles, 1 one wide CTA per SM (48 KB stages), 2 (default) two per
+// packed path: QBG_GEMM_WIDE in the environment, 0 leaves every product to the
+// staged kernel, 1 one packed CTA per SM (48 KB stages), 2 (default) two per
 // SM (24 KB stages; C2 factor phase 28.1 -> 26.7 ms against 1)
 std::atomic<int> g_pkw_mode{[] {
   const char* e = std::getenv("QBG_GEMM_WIDE");
